@@ -40,6 +40,7 @@ struct PpbEmitView {
   uint32_t* slot_segs;  // [P * K] segments of each beam
   uint32_t* slot_off;   // [P * K] exclusive prefix inside the photon
   uint32_t* photon_segs;// [P]
+  float* reach;         // [P * K] the farthest of each beam's transmittance distances
   uint32_t photons, K;
   float radius;
   uint32_t seed, pass;
@@ -106,10 +107,14 @@ __global__ void __launch_bounds__(128) ppb_emit_kernel(GridView g, SceneView s, 
       sl[3] = d.x; sl[4] = d.y; sl[5] = d.z;
       sl[6] = tmax;
       sl[7] = power.x; sl[8] = power.y; sl[9] = power.z;
+      float reach = 0.0f;
       for (int i = 0; i < kBeamDists; ++i) {
         float t;
-        sl[10 + i] = free_flight(g, s, o, d, rng, t, lookups, cells) ? t : kEscaped;
+        const float e = free_flight(g, s, o, d, rng, t, lookups, cells) ? t : kEscaped;
+        sl[10 + i] = e;
+        reach = fmaxf(reach, e);
       }
+      v.reach[(size_t)p * v.K + beams] = reach;
       uint32_t ns = segments_of(tmax, v.radius);
       v.slot_segs[(size_t)p * v.K + beams] = ns;
       v.slot_off[(size_t)p * v.K + beams] = seg_total;
@@ -230,16 +235,129 @@ __device__ __forceinline__ void segment_box(float4 A, float4 B, float4& lo, floa
   hi = make_float4(fmaxf(pa.x + e.x, pb.x + e.x), fmaxf(pa.y + e.y, pb.y + e.y), fmaxf(pa.z + e.z, pb.z + e.z), 0.f);
 }
 
-// The segments in leaf order: leaf i holds segment order[i].
-__global__ void ppb_leaf_order_kernel(const uint32_t* __restrict__ order, const float4* __restrict__ seg_a,
-                                      const float4* __restrict__ seg_b, const uint32_t* __restrict__ seg_beam,
-                                      uint32_t n, float4* __restrict__ leaf_a, float4* __restrict__ leaf_b,
-                                      uint32_t* __restrict__ leaf_beam) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t sid = order[i];
-    leaf_a[i] = seg_a[sid];
-    leaf_b[i] = seg_b[sid];
-    leaf_beam[i] = seg_beam[sid];
+// Boxes that cover `leaves` leaves, 2^log2_per_box leaves a box.
+__device__ __forceinline__ uint32_t boxes_above(uint32_t leaves, uint32_t log2_per_box) {
+  return (uint32_t)(((uint64_t)leaves + (1ull << log2_per_box) - 1ull) >> log2_per_box);
+}
+
+// Union of a warp's boxes, in every lane.
+__device__ __forceinline__ void warp_box(float4& lo, float4& hi) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
+    lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
+    lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
+    hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
+    hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
+    hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
+  }
+}
+
+// Which leaves can contribute to any pixel, 32 leaves (a cluster of the
+// Morton order) a warp: a segment past the farthest of its beam's 16
+// transmittance distances has none of them left, and where every majorant
+// cell its box touches is zero the density at the closest point is; both
+// factors of the estimate are then exactly 0.  A cell's majorant bounds the
+// trilinear lookups inside it.  The points looked up lie within the radius of
+// the segment; its box is grown by that, and by a hundredth of a cell against
+// the rounding of the cell index.
+struct LiveView {
+  const uint32_t* order;
+  const float4* seg_a;
+  const float4* seg_b;
+  const uint32_t* seg_beam;
+  const float* reach;
+  const float* maj;  // a pyramid level
+  int mnb[3];
+  f3 b0, icell;
+};
+__device__ __forceinline__ bool segment_meets_density(const LiveView& v, float4 A, float4 B) {
+  const float r = A.w;
+  const float l[3] = {(fminf(A.x, B.x) - r - v.b0.x) * v.icell.x, (fminf(A.y, B.y) - r - v.b0.y) * v.icell.y,
+                      (fminf(A.z, B.z) - r - v.b0.z) * v.icell.z};
+  const float h[3] = {(fmaxf(A.x, B.x) + r - v.b0.x) * v.icell.x, (fmaxf(A.y, B.y) + r - v.b0.y) * v.icell.y,
+                      (fmaxf(A.z, B.z) + r - v.b0.z) * v.icell.z};
+  int c0[3], c1[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float top = (float)(v.mnb[a] - 1);
+    c0[a] = (int)clampf(floorf(l[a] - 0.01f), 0.0f, top);
+    c1[a] = (int)clampf(floorf(h[a] + 0.01f), 0.0f, top);
+  }
+  if ((c1[0] - c0[0] + 1) * (c1[1] - c0[1] + 1) * (c1[2] - c0[2] + 1) > 64) return true;  // not worth the walk
+  for (int z = c0[2]; z <= c1[2]; ++z)
+    for (int y = c0[1]; y <= c1[1]; ++y)
+      for (int x = c0[0]; x <= c1[0]; ++x)
+        if (!(__ldg(v.maj + ((size_t)x + (size_t)v.mnb[0] * ((size_t)y + (size_t)v.mnb[1] * z))) == 0.0f)) return true;
+  return false;
+}
+__global__ void __launch_bounds__(256) ppb_live_kernel(const __grid_constant__ LiveView v, uint32_t n,
+                                                       uint32_t* __restrict__ masks, uint32_t* __restrict__ counts) {
+  const uint32_t lane = threadIdx.x & 31u, c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= (n + 31u) / 32u) return;  // warp-uniform
+  const uint32_t i = c * 32u + lane;
+  bool live = false;
+  if (i < n) {
+    const uint32_t sid = v.order[i];
+    const float4 B = v.seg_b[sid];
+    live = v.reach[v.seg_beam[sid]] >= B.w && segment_meets_density(v, v.seg_a[sid], B);
+  }
+  const uint32_t m = __ballot_sync(0xffffffffu, live);
+  if (lane == 0) {
+    masks[c] = m;
+    counts[c] = __popc(m);
+  }
+}
+
+// The gather's leaves: the live ones in leaf order, segments and boxes side
+// by side with their neighbours'.
+struct GatherLeaves {
+  float4* a;
+  float4* b;
+  float4* lo;
+  float4* hi;
+  uint32_t* beam;
+};
+__global__ void __launch_bounds__(256) ppb_compact_kernel(const uint32_t* __restrict__ order,
+                                                          const float4* __restrict__ seg_a,
+                                                          const float4* __restrict__ seg_b,
+                                                          const uint32_t* __restrict__ seg_beam,
+                                                          const float4* __restrict__ leaf_lo,
+                                                          const float4* __restrict__ leaf_hi, uint32_t n,
+                                                          const uint32_t* __restrict__ masks,
+                                                          const uint32_t* __restrict__ offsets, GatherLeaves out) {
+  const uint32_t lane = threadIdx.x & 31u, c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= (n + 31u) / 32u) return;  // warp-uniform
+  const uint32_t m = masks[c];
+  if (!((m >> lane) & 1u)) return;
+  const uint32_t i = c * 32u + lane, sid = order[i], at = offsets[c] + __popc(m & ((1u << lane) - 1u));
+  out.a[at] = seg_a[sid];
+  out.b[at] = seg_b[sid];
+  out.beam[at] = seg_beam[sid];
+  out.lo[at] = leaf_lo[i];
+  out.hi[at] = leaf_hi[i];
+}
+
+// A cluster level: box c over boxes [32 c, 32 c + 32) of the level below,
+// which has ceil(*leaves / per_box) of them (the live leaves' count is on
+// the device; the launch covers the most there can be).
+__global__ void __launch_bounds__(256) ppb_cluster_kernel(const float4* __restrict__ lo_in,
+                                                          const float4* __restrict__ hi_in,
+                                                          const uint32_t* __restrict__ leaves, uint32_t log2_per_box,
+                                                          float4* __restrict__ clo, float4* __restrict__ chi) {
+  const uint32_t n = boxes_above(*leaves, log2_per_box);
+  const uint32_t lane = threadIdx.x & 31u, c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= (n + 31u) / 32u) return;  // warp-uniform
+  const uint32_t i = c * 32u + lane;
+  float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+  if (i < n) {
+    lo = lo_in[i];
+    hi = hi_in[i];
+  }
+  warp_box(lo, hi);
+  if (lane == 0) {
+    clo[c] = lo;
+    chi[c] = hi;
   }
 }
 
@@ -297,48 +415,41 @@ __global__ void lbvh_refit_kernel(const float4* __restrict__ seg_a, const float4
 // ---------------------------------------------------------------------------
 // gather
 // ---------------------------------------------------------------------------
-// What the gather reads: the segments in the LBVH's leaf order (leaf i
-// holds segment order[i]), the leaf boxes, and per internal node its own
-// packed node (low corner, left child bits) (high corner, right child bits)
-// followed by its two children's (a child leaf: its box), so that one round
-// of loads covers two levels of the tree.
+// Boxes over 32 consecutive leaves of the Morton order (level 0), over 32 of
+// those (level 1), ... up to the first level of at most 32 boxes.
+constexpr int kClusterLevels = 6;  // 32^6 leaves > 2^26
+struct ClusterLayout {
+  uint32_t count[kClusterLevels];  // boxes of each level when every leaf is live
+  uint32_t first[kClusterLevels];  // the level's first box in the arrays
+  int levels;
+  uint32_t total;
+};
+static ClusterLayout cluster_layout(uint32_t leaves) {
+  ClusterLayout c{};
+  uint32_t n = leaves;
+  do {
+    n = (n + 31u) / 32u;
+    c.count[c.levels] = n;
+    c.first[c.levels++] = c.total;
+    c.total += n;
+  } while (n > 32u && c.levels < kClusterLevels);
+  return c;
+}
+
+// What the gather reads: the live segments in the LBVH's leaf order, their
+// boxes and the cluster boxes above them, the beam slots and each pixel's
+// camera free flights.
 struct PpbGatherView {
-  const float4* seg_a;
-  const float4* seg_b;
-  const uint32_t* seg_beam;
+  GatherLeaves leaf;
+  const uint32_t* n_live;
   const float* slots;
-  const float4* leaf_lo;
-  const float4* leaf_hi;
-  const float4* node2;
-  int n;
+  const float4* cluster_lo;
+  const float4* cluster_hi;
+  float* cam_dist;
+  ClusterLayout cl;
+  float radius;
   uint32_t seed, pass;
 };
-
-// Two levels of the LBVH per internal node b: node2[6b..6b+1] = b's packed
-// node, [6b+2..6b+3] and [6b+4..6b+5] = its left and right child's packed
-// node, or the child leaf's box (its leaf id stays in b's child bits).
-__global__ void lbvh_node2_kernel(const float4* __restrict__ node_pk, const float4* __restrict__ leaf_lo,
-                                  const float4* __restrict__ leaf_hi, uint32_t internal,
-                                  float4* __restrict__ node2) {
-  for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < internal; b += gridDim.x * blockDim.x) {
-    const float4 q0 = node_pk[2 * (size_t)b], q1 = node_pk[2 * (size_t)b + 1];
-    float4* o = node2 + 6 * (size_t)b;
-    o[0] = q0;
-    o[1] = q1;
-    const uint32_t ch[2] = {__float_as_uint(q0.w), __float_as_uint(q1.w)};
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const uint32_t c = ch[k];
-      if (c & kLeafBit) {
-        o[2 + 2 * k] = leaf_lo[c & ~kLeafBit];
-        o[3 + 2 * k] = leaf_hi[c & ~kLeafBit];
-      } else {
-        o[2 + 2 * k] = node_pk[2 * (size_t)c];
-        o[3 + 2 * k] = node_pk[2 * (size_t)c + 1];
-      }
-    }
-  }
-}
 
 // Ray-box overlap of [t0, t1] with the slab interval.
 __device__ __forceinline__ bool ray_box(f3 o, f3 inv, float t0, float t1, float4 lo, float4 hi) {
@@ -350,175 +461,493 @@ __device__ __forceinline__ bool ray_box(f3 o, f3 inv, float t0, float t1, float4
   return tn <= tf;
 }
 
+// Camera ray of a crop pixel clipped to the cloud's box; false: it sees the
+// sky alone.
+__device__ __forceinline__ bool gather_ray(const SceneView& s, const CamView& cam, const PassView& pv, uint32_t cx,
+                                           uint32_t cy, f3& o, f3& rd, float& t_in, float& t_out) {
+  camera_ray(cam, (int)(pv.x0 + cx), (int)(pv.y0 + cy), o, rd);
+  float tmin, tmax;
+  if (!slab(o, rd, s.b0, s.b1, tmin, tmax) || tmax < 0.0f || !(s.ds > 0.0f)) return false;
+  t_in = fmaxf(tmin, 0.0f);
+  t_out = tmax;
+  return true;
+}
+
+// Ascending order of 16 values (Batcher's bitonic sort, 80 exchanges): how
+// many of them are at least x is then a binary search.
+__device__ __forceinline__ void sort16(float (&v)[kBeamDists]) {
+#pragma unroll
+  for (int size = 2; size <= kBeamDists; size *= 2)
+#pragma unroll
+    for (int stride = size / 2; stride > 0; stride /= 2)
+#pragma unroll
+      for (int i = 0; i < kBeamDists; ++i) {
+        const int j = i ^ stride;
+        if (j < i) continue;
+        const float a = fminf(v[i], v[j]), b = fmaxf(v[i], v[j]);
+        v[i] = (i & size) == 0 ? a : b;
+        v[j] = (i & size) == 0 ? b : a;
+      }
+}
+
+// The 16 free flights along each pixel's camera ray, stored in ascending
+// order.  One thread a pixel; its flights follow one another in one loop
+// over tentative collisions, so lanes whose flights end early go on with
+// their next one instead of waiting for the warp's longest.
+__global__ void __launch_bounds__(128) ppb_camera_kernel(GridView g, SceneView s, CamView cam, PassView pv,
+                                                         PpbGatherView v, Counters cnt) {
+  const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t lookups = 0, cells = 0;
+  if (id < pv.cw * pv.ch) {
+    const uint32_t cy = id / pv.cw, cx = id - cy * pv.cw;
+    f3 o, rd;
+    float t_in, t_out;
+    if (gather_ray(s, cam, pv, cx, cy, o, rd, t_in, t_out)) {
+      const uint32_t pix = (pv.y0 + cy) * pv.width + pv.x0 + cx;
+      const f3 entry = along(o, rd, t_in);
+      Rng rng = rng_pcg(v.seed ^ kGatherSalt, pix, v.pass);
+      float d[kBeamDists];
+#pragma unroll
+      for (int i = 0; i < kBeamDists; ++i) d[i] = kEscaped;
+      Track tr;
+      int i = 0;
+      bool fresh = true;
+      while (i < kBeamDists) {
+        if (fresh) track_init(tr, g, s, g.majorants, entry, rd, cells);
+        fresh = false;
+        float tau = -vlog(rng_next(rng));
+        bool ended = true;
+        float t = kEscaped;
+        if (track_walk(tr, g, g.majorants, s.k_sigma, tau, cells, 0xFFFFFFFFu) == kCandidate) {
+          const float rho = density_at(g, s, along(entry, rd, tr.t));
+          ++lookups;
+          if (rng_next(rng) * tr.m < rho) t = tr.t;
+          else ended = lookups + cells > kPathWorkCap;  // runaway guard (non-finite input)
+        }
+        if (ended) {
+#pragma unroll
+          for (int k = 0; k < kBeamDists; ++k)
+            if (k == i) d[k] = t;  // constant indices: the values stay in registers
+          ++i;
+          fresh = true;
+        }
+      }
+      sort16(d);
+      float4* out = reinterpret_cast<float4*>(v.cam_dist + (size_t)id * kBeamDists);
+#pragma unroll
+      for (int k = 0; k < kBeamDists / 4; ++k) out[k] = make_float4(d[4 * k], d[4 * k + 1], d[4 * k + 2], d[4 * k + 3]);
+    }
+  }
+  flush_counters(cnt, 0ull, lookups, 0, cells);
+}
+
+// A pixel tile's view of the scene, for finding the tile's pixels whose rays
+// can meet a box.  A point p lies on the ray of the pixel (a, b) away from
+// the tile's centre where A(p - apex) = a W(p - apex) and B(p - apex) = b
+// W(p - apex), with the three linear forms of the camera's basis.  The box
+// is grown by `grow` (1e-5 of the scene's coordinates: the rounding of the
+// exact ray-box test) and the pixel range by `slack` (1/32 pixel and the
+// forms' own rounding, which grows with the tile's distance from the image
+// centre), so every pixel whose ray meets the box is in the range.
+struct TileView {
+  f3 apex, W, A, B;
+  float grow, slack, far;
+};
+__device__ __forceinline__ TileView tile_view(const CamView& c, const SceneView& s, int x0, int y0, int w, int h) {
+  const f3 F = c.fwd * c.near_plane, R = c.right * c.px, U = -(c.up * c.py);
+  const f3 ru = cross(R, U), uf = cross(U, F), fr = cross(F, R);
+  const float inv = 1.0f / dot(F, ru);
+  TileView t;
+  t.apex = c.pos;
+  t.W = ru * inv;
+  // pixels relative to the tile's centre
+  const float ac = (float)(x0 - c.hw) + 0.5f * (float)(w - 1), bc = (float)(y0 - c.hh) + 0.5f * (float)(h - 1);
+  t.A = uf * inv - t.W * ac;
+  t.B = fr * inv - t.W * bc;
+  t.far = INFINITY;
+  t.slack = 0.03125f + 4e-6f * (fabsf(ac) + fabsf(bc));
+  t.grow = 1e-5f * fmaxf(fmaxf(fmaxf(fabsf(c.pos.x), fabsf(c.pos.y)), fabsf(c.pos.z)),
+                         fmaxf(fmaxf(fmaxf(fabsf(s.b0.x), fabsf(s.b0.y)), fabsf(s.b0.z)),
+                               fmaxf(fmaxf(fabsf(s.b1.x), fabsf(s.b1.y)), fabsf(s.b1.z))));
+  return t;
+}
+// The pixels (bit x + kW y) of the tile that the box may cover: all of them
+// where the box reaches the camera's plane or a form is not finite.
+template <uint32_t kW, uint32_t kH>
+__device__ __forceinline__ uint32_t tile_pixels(const TileView& t, float4 lo, float4 hi) {
+  const float cx = 0.5f * (lo.x + hi.x), cy = 0.5f * (lo.y + hi.y), cz = 0.5f * (lo.z + hi.z);
+  const float ex = hi.x - cx + t.grow, ey = hi.y - cy + t.grow, ez = hi.z - cz + t.grow;
+  const float rx = cx - t.apex.x, ry = cy - t.apex.y, rz = cz - t.apex.z;
+  const float wc = fmaf(t.W.x, rx, fmaf(t.W.y, ry, t.W.z * rz));
+  const float we = fmaf(fabsf(t.W.x), ex, fmaf(fabsf(t.W.y), ey, fabsf(t.W.z) * ez));
+  const float ac = fmaf(t.A.x, rx, fmaf(t.A.y, ry, t.A.z * rz));
+  const float ae = fmaf(fabsf(t.A.x), ex, fmaf(fabsf(t.A.y), ey, fabsf(t.A.z) * ez));
+  const float bc = fmaf(t.B.x, rx, fmaf(t.B.y, ry, t.B.z * rz));
+  const float be = fmaf(fabsf(t.B.x), ex, fmaf(fabsf(t.B.y), ey, fabsf(t.B.z) * ez));
+  const float near_w = wc - we;
+  if (near_w > t.far) return 0u;  // behind every ray's end
+  constexpr uint32_t kRows = 1u | (kH > 1u ? 1u << kW : 0u) | (kH > 2u ? 1u << 2u * kW | 1u << 3u * kW : 0u);
+  static_assert((kH == 1u || kH == 2u || kH == 4u) && kW * kH <= 32u, "tile shapes");
+  constexpr uint32_t kAll = (kW * kH == 32u) ? 0xFFFFFFFFu : (1u << (kW * kH)) - 1u;
+  const float in = 1.0f / near_w, fn = 1.0f / (wc + we);
+  constexpr float hx = 0.5f * (float)(kW - 1u), hy = 0.5f * (float)(kH - 1u);
+  const float a0 = ac - ae, a1 = ac + ae, b0 = bc - be, b1 = bc + be;
+  const float x0 = ceilf(a0 * (a0 < 0.0f ? in : fn) + (hx - t.slack));
+  const float x1 = floorf(a1 * (a1 > 0.0f ? in : fn) + (hx + t.slack));
+  const float y0 = ceilf(b0 * (b0 < 0.0f ? in : fn) + (hy - t.slack));
+  const float y1 = floorf(b1 * (b1 > 0.0f ? in : fn) + (hy + t.slack));
+  if (!(near_w > 0.0f) || !(x0 == x0 && x1 == x1 && y0 == y0 && y1 == y1)) return kAll;
+  if (x1 < 0.0f || y1 < 0.0f || x0 > (float)(kW - 1u) || y0 > (float)(kH - 1u) || x1 < x0 || y1 < y0) return 0u;
+  const uint32_t xa = (uint32_t)fmaxf(x0, 0.0f), xb = (uint32_t)fminf(x1, (float)(kW - 1u));
+  const uint32_t ya = (uint32_t)fmaxf(y0, 0.0f), yb = (uint32_t)fminf(y1, (float)(kH - 1u));
+  const uint32_t row = (2u << xb) - (1u << xa);
+  return row * ((kRows << (kW * ya)) & (kRows >> (kW * (kH - 1u - yb))));
+}
+
 // Beam x beam (1D) estimate of one segment (accumulateRadiance,
-// PPB_PE.comp:362-404, with the fixes named at the top of the file); A, B:
-// its endpoints (with the radius and the offset from the beam origin).
-__device__ __forceinline__ f3 beam_contribution(const GridView& g, const SceneView& s, const PpbGatherView& v,
-                                                float4 A, float4 B, uint32_t beam, f3 o, f3 rd, float t_in,
-                                                float t_out, const float* cam_d, uint32_t& lookups) {
-  f3 pa = mk(A.x, A.y, A.z), pb = mk(B.x, B.y, B.z);
-  float r = A.w;
-  f3 ax = pb - pa;
-  float segl = length(ax);
-  f3 zero = mk(0.f, 0.f, 0.f);
-  if (!(segl > 0.0f)) return zero;
-  f3 bd = mk(ax.x / segl, ax.y / segl, ax.z / segl);
+// PPB_PE.comp:362-404, with the fixes named at the top of the file), in two
+// steps.  The first, for every (ray, segment) pair: the closest points of
+// the camera ray (o, rd) and the segment (start pa, unit direction bd,
+// length segl), at t along the ray and sb along the segment; false where the
+// pair contributes nothing.  The distance is compared squared, with a margin
+// over the rounding of the square root; the second step decides with it.
+__device__ __forceinline__ bool beam_closest(f3 pa, float r, f3 bd, float segl, f3 o, f3 rd, float t_in, float t_far,
+                                             float& t, float& sb) {
+  if (!(segl > 0.0f)) return false;
   float b = dot(rd, bd);
   float den = 1.0f - b * b;
-  if (!(den > 1e-6f)) return zero;  // (nearly) parallel
+  if (!(den > 1e-6f)) return false;  // (nearly) parallel
   f3 w0 = o - pa;
   float dw = dot(rd, w0), ew = dot(bd, w0);
-  float t = (b * ew - dw) / den;
-  float sb = ew + t * b;
-  if (t < t_in || t > t_out || sb < 0.0f || sb > segl) return zero;
+  t = (b * ew - dw) / den;
+  sb = ew + t * b;
+  if (t < t_in || t > t_far || sb < 0.0f || sb > segl) return false;
+  const f3 e = along(o, rd, t) - along(pa, bd, sb);
+  const float r2 = r * r;
+  return dot(e, e) < r2 * 1.000001f || !(r2 > 1e-30f);
+}
+
+// The second step: the contribution of a pair the first one kept.  off: the
+// segment's distance from its beam's origin; dist: the pixel's 16 ascending
+// camera flights.
+__device__ __forceinline__ f3 beam_contribution(const GridView& g, const SceneView& s, const float* __restrict__ sl,
+                                                f3 pa, float r, f3 bd, float off, f3 o, f3 rd, float t_in, float t,
+                                                float sb, const float* __restrict__ dist16, uint32_t& lookups) {
   f3 xc = along(o, rd, t);
   f3 xb = along(pa, bd, sb);
   float dist = length(xc - xb);
-  if (!(dist < r)) return zero;
+  if (!(dist < r)) return mk(0.f, 0.f, 0.f);
+  float b = dot(rd, bd);
+  float den = 1.0f - b * b;
   float u = dist / r;
   float q = 1.0f - u * u;
   float kern = ((0.9375f * q) * q) / r;  // 15/16 (1 - u^2)^2 / r
   float rho = density_at(g, s, xc);
   ++lookups;
   float sigma_s = (s.albedo * s.k_sigma) * rho;
-  const float* sl = v.slots + (size_t)beam * kSlotFloats;
-  float sbeam = sb + B.w;  // distance from the beam origin
-  uint32_t cb = 0, cc = 0;
-  float tc = t - t_in;
-  for (int i = 0; i < kBeamDists; ++i) {
-    cb += sl[10 + i] >= sbeam ? 1u : 0u;
-    cc += cam_d[i] >= tc ? 1u : 0u;
+  float sbeam = sb + off;  // distance from the beam origin
+  const float2* s2 = reinterpret_cast<const float2*>(sl);  // slots are 112 B: 8-byte aligned pairs
+  uint32_t cb = 0;
+#pragma unroll
+  for (int i = 0; i < kBeamDists / 2; ++i) {
+    const float2 e = __ldg(s2 + 5 + i);
+    cb += (e.x >= sbeam ? 1u : 0u) + (e.y >= sbeam ? 1u : 0u);
   }
+  const float2 p0 = __ldg(s2 + 3), p12 = __ldg(s2 + 4);  // (length, power r), (power g, power b)
+  float tc = t - t_in;
+  uint32_t below = 0;  // camera flights shorter than tc
+#pragma unroll
+  for (uint32_t k = 8; k > 0; k >>= 1)
+    if (__ldg(dist16 + below + k - 1) < tc) below += k;
+  if (below == 15u && __ldg(dist16 + 15) < tc) below = 16u;
+  uint32_t cc = (uint32_t)kBeamDists - below;
   float tb = (float)cb * (1.0f / kBeamDists), tcam = (float)cc * (1.0f / kBeamDists);
   float ph = hg_pdf(s.ph, dot(bd, -rd));
   float w = ((((kern * sigma_s) * tcam) * tb) * ph) / sqrtf(den);
-  return mk(sl[7] * w, sl[8] * w, sl[9] * w);
+  return mk(p0.y * w, p12.x * w, p12.y * w);
 }
 
-// Per-pixel gather with a warp-coherent traversal: a warp takes an 8x4
-// pixel tile and walks the tree once for all its rays.  Each stack entry
-// carries the mask of lanes whose rays hit the parent, and a lane tests and
-// evaluates exactly the nodes and leaves its own single-ray depth-first walk
-// would, in the same order (so its sum is the same); node data are loaded
-// once for the warp (one broadcast transaction instead of one per lane).
-// A visit of internal node b loads b's and its children's boxes together
-// (node2) and tests both levels: the right child's part goes onto the stack
-// first (its leaf, or its two children with the lanes that hit it), then
-// the left child's (its right child), and the walk continues at the left
-// child's left child (or the left leaf) — the binary walk's order.
+// Per-pixel gather.  A warp takes a tile of P pixels and finds the leaves
+// whose boxes its rays may meet by descending the 32-wide cluster boxes, one
+// lane a box (coalesced loads; the box's pixel range in the tile by three
+// linear forms).  The kept leaves' segments go to shared memory with their
+// directions and lengths worked out once a tile and the pixels they may
+// cover.  The (leaf, pixel) pairs of a batch are listed and tested 32 at a
+// time, one lane a pair: the exact box test (the single-ray walk of the LBVH
+// visits exactly the leaves whose boxes the ray meets, since a ray that
+// meets a box meets every box around it), and the closest points.  The pairs
+// that contribute - about one box hit in five - are queued and evaluated 32
+// at a time, again one lane a pair.  A pixel adds its pairs' contributions
+// in queue order, which is ascending leaf order: the order of the
+// depth-first walk, so the sums are the same floats.
+//
+// Bound by instruction issue (0.75 of the slots at 24 warps an SM), most of
+// it the evaluation's divisions, square roots and gathers.  1280x720, 60,741
+// photons, 9.6 M segments of radius 0.015: 27.5 ms for 1.82 G box hits, of
+// 5.48 G before the leaves and ray ends that give exactly 0 were left out
+// (ppb_live_kernel, t_far; 71.9 ms).  The same walk with one lane a pixel
+// for the closest points and the evaluation, 12 lanes of 32 at work, took
+// 129 ms.
 constexpr int kGatherThreads = 128;
-constexpr int kGatherStack2 = 128;  // up to 3 entries a visit of two levels (depth <= 64)
+constexpr int kGatherWarps = kGatherThreads / 32;
+constexpr int kLeafBatch = 64;  // leaf slots of a warp; a batch is tested once more than 32 are filled
+__host__ __device__ constexpr uint32_t gather_w(int P) { return P == 32 ? 8u : P >= 8 ? 4u : 2u; }
 
-__global__ void __launch_bounds__(kGatherThreads) ppb_gather_kernel(GridView g, SceneView s, CamView cam, PassView pv,
-                                                                    PpbGatherView v, double* __restrict__ sum,
-                                                                    Counters cnt,
+template <int P>
+struct __align__(16) GatherWarp {
+  float4 leaf[kLeafBatch][4];  // (box lo, offset) (box hi, beam) (start, radius) (direction, length)
+  float4 ray[P][3];            // (origin, t_in) (direction, t_far) (1 / direction, t_box)
+  float2 q_t[64];              // queued pairs: (t, sb)
+  uint32_t q_id[64];           // leaf slot << 5 | pixel
+  uint32_t pixels[kLeafBatch]; // the tile's pixels a leaf's box may cover
+  float c[3][32];              // contributions of a group of pairs
+  uint32_t own[P];             // each pixel's pairs in the group
+  uint32_t mask[kClusterLevels], base[kClusterLevels];
+  uint16_t pair[32 * P];       // the pairs of 32 leaves: leaf slot << 5 | pixel
+};
+
+template <int P>
+__global__ void __launch_bounds__(kGatherThreads, 6) ppb_gather_kernel(const __grid_constant__ GridView g,
+                                                                    const __grid_constant__ SceneView s,
+                                                                    const __grid_constant__ CamView cam,
+                                                                    const __grid_constant__ PassView pv,
+                                                                    const __grid_constant__ PpbGatherView v,
+                                                                    double* __restrict__ sum, Counters cnt,
                                                                     unsigned long long* __restrict__ evaluated) {
-  __shared__ uint2 s_stack[kGatherThreads / 32][kGatherStack2];
-  const uint32_t lane = threadIdx.x & 31u;
+  constexpr uint32_t kW = gather_w(P), kH = (uint32_t)P / kW;
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  GatherWarp<P>& w = reinterpret_cast<GatherWarp<P>*>(s_raw)[threadIdx.x >> 5];
+  const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
   const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t tiles_x = (pv.cw + 7u) / 8u;
-  const uint32_t cx = (wid % tiles_x) * 8u + (lane & 7u), cy = (wid / tiles_x) * 4u + (lane >> 3);
-  const bool valid = cx < pv.cw && cy < pv.ch;
-  uint32_t lookups = 0, cells = 0, segs = 0;
-  uint32_t pix = 0;
-  f3 o = mk(0.f, 0.f, 0.f), rd = mk(0.f, 0.f, 1.f), L = mk(0.f, 0.f, 0.f);
-  float t_in = 0.0f, t_out = 0.0f;
-  float cam_d[kBeamDists];
+  const uint32_t tiles_x = (pv.cw + kW - 1u) / kW;
+  const uint32_t tx0 = (wid % tiles_x) * kW, ty0 = (wid / tiles_x) * kH;
+  const uint32_t cx = tx0 + lane % kW, cy = ty0 + lane / kW;  // lane p < P owns pixel p of the tile
+  const bool valid = lane < (uint32_t)P && cx < pv.cw && cy < pv.ch;
+  uint32_t lookups = 0, segs = 0;
+  f3 L = mk(0.f, 0.f, 0.f);
   bool trav = false;
+  float depth = -INFINITY;  // W of the tile's farthest ray end
+  const uint32_t n = *v.n_live;
+  TileView view = tile_view(cam, s, (int)(pv.x0 + tx0), (int)(pv.y0 + ty0), (int)kW, (int)kH);
   if (valid) {
-    int x = (int)(pv.x0 + cx), y = (int)(pv.y0 + cy);
-    pix = (uint32_t)y * pv.width + (uint32_t)x;
-    camera_ray(cam, x, y, o, rd);
-    float tmin, tmax;
-    if (!slab(o, rd, s.b0, s.b1, tmin, tmax) || tmax < 0.0f || !(s.ds > 0.0f)) {
+    f3 o, rd;
+    float t_in, t_out;
+    if (!gather_ray(s, cam, pv, cx, cy, o, rd, t_in, t_out)) {
       L = sky(s, rd);
     } else {
-      t_in = fmaxf(tmin, 0.0f);
-      t_out = tmax;
-      f3 entry = along(o, rd, t_in);
-      Rng rng = rng_pcg(v.seed ^ kGatherSalt, pix, v.pass);
-      for (int i = 0; i < kBeamDists; ++i) {
-        float t;
-        cam_d[i] = free_flight(g, s, entry, rd, rng, t, lookups, cells) ? t : kEscaped;
-      }
+      const float4* d = reinterpret_cast<const float4*>(v.cam_dist + (size_t)(cy * pv.cw + cx) * kBeamDists);
+      const float through = t_out - t_in;
       uint32_t cexit = 0;
-      for (int i = 0; i < kBeamDists; ++i) cexit += cam_d[i] >= (t_out - t_in) ? 1u : 0u;
-      L = sky(s, rd) * ((float)cexit * (1.0f / kBeamDists));
-      trav = v.n > 0;
-    }
-  }
-  uint32_t active = __ballot_sync(0xffffffffu, trav);
-  if (active) {
-    uint2* stk = s_stack[threadIdx.x >> 5];
-    const f3 inv = mk(1.0f / rd.x, 1.0f / rd.y, 1.0f / rd.z);
-    int sp = 0;  // warp-uniform, as are node and active
-    uint32_t node = v.n == 1 ? (0u | kLeafBit) : 0u;
-    while (true) {
-      const bool mine = (active >> lane) & 1u;
-      if (node & kLeafBit) {
-        // the leaf's box and its segment (leaf order) in one round of loads
-        const uint32_t lf = node & ~kLeafBit;
-        const float4 lo = v.leaf_lo[lf], hi = v.leaf_hi[lf];
-        const float4 A = v.seg_a[lf], B = v.seg_b[lf];
-        const uint32_t beam = v.seg_beam[lf];
-        if (mine && ray_box(o, inv, t_in, t_out, lo, hi)) {
-          L = L + beam_contribution(g, s, v, A, B, beam, o, rd, t_in, t_out, cam_d, lookups);
-          ++segs;
-        }
-      } else {
-        const float4* q = v.node2 + 6 * (size_t)node;
-        const float4 q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4], q5 = q[5];
-        const uint32_t hit = __ballot_sync(0xffffffffu, mine && ray_box(o, inv, t_in, t_out, q0, q1));
-        if (hit) {
-          const bool hb = (hit >> lane) & 1u;
-          const uint32_t l = __float_as_uint(q0.w), r = __float_as_uint(q1.w);
-          // at most 3 pushes a visit of two levels: below kGatherStack2 for
-          // depth <= 64 (30-bit keys + index bits); the guard only keeps a
-          // deeper tree in bounds
-          if (r & kLeafBit) {
-            if (sp < kGatherStack2) {
-              if (lane == 0) stk[sp] = make_uint2(r, hit);
-              ++sp;
-            }
-          } else {
-            const uint32_t h1 = __ballot_sync(0xffffffffu, hb && ray_box(o, inv, t_in, t_out, q4, q5));
-            if (h1 && sp + 2 <= kGatherStack2) {
-              if (lane == 0) {
-                stk[sp] = make_uint2(__float_as_uint(q5.w), h1);
-                stk[sp + 1] = make_uint2(__float_as_uint(q4.w), h1);
-              }
-              sp += 2;
-            }
-          }
-          if (l & kLeafBit) {
-            node = l;
-            active = hit;
-            continue;
-          }
-          const uint32_t h0 = __ballot_sync(0xffffffffu, hb && ray_box(o, inv, t_in, t_out, q2, q3));
-          if (h0) {
-            if (sp < kGatherStack2) {
-              if (lane == 0) stk[sp] = make_uint2(__float_as_uint(q3.w), h0);
-              ++sp;
-            }
-            node = __float_as_uint(q2.w);
-            active = h0;
-            continue;
-          }
-        }
+#pragma unroll
+      for (int i = 0; i < kBeamDists / 4; ++i) {
+        const float4 q = d[i];
+        cexit += (q.x >= through ? 1u : 0u) + (q.y >= through ? 1u : 0u) + (q.z >= through ? 1u : 0u) +
+                 (q.w >= through ? 1u : 0u);
       }
-      if (sp == 0) break;
-      --sp;
-      __syncwarp();
-      const uint2 e = stk[sp];
-      __syncwarp();
-      node = e.x;
-      active = e.y;
+      L = sky(s, rd) * ((float)cexit * (1.0f / kBeamDists));
+      trav = n > 0u;
+      // past the farthest flight (d[3].w) the camera transmittance is 0 (the
+      // margin is over the rounding of t - t_in); the boxes are looked for
+      // some radii further, as a closest point may lie before its box
+      const float t_far = fminf(t_out, (t_in + d[kBeamDists / 4 - 1].w) * 1.0001f);
+      const float t_box = fminf(t_out, t_far + 8.0f * v.radius);
+      depth = fmaf(view.W.x, fmaf(t_box, rd.x, o.x - view.apex.x),
+                   fmaf(view.W.y, fmaf(t_box, rd.y, o.y - view.apex.y),
+                        view.W.z * fmaf(t_box, rd.z, o.z - view.apex.z)));
+      w.ray[lane][0] = make_float4(o.x, o.y, o.z, t_in);
+      w.ray[lane][1] = make_float4(rd.x, rd.y, rd.z, t_far);
+      w.ray[lane][2] = make_float4(1.0f / rd.x, 1.0f / rd.y, 1.0f / rd.z, t_box);
     }
   }
-  if (valid) write_result(pv, sum, pix, L);
-  flush_counters(cnt, valid ? 1ull : 0ull, lookups, 0, cells);
+  const uint32_t rays = __ballot_sync(0xffffffffu, trav);
+  if (rays) {
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) depth = fmaxf(depth, __shfl_xor_sync(0xffffffffu, depth, k));
+    view.far = depth;
+    const int top = v.cl.levels - 1;
+    int lev = top;  // warp-uniform, as are filled and the masks
+    uint32_t filled = 0;
+    bool done = false;
+    {
+      bool see = false;
+      if (lane < boxes_above(n, 5u * (uint32_t)v.cl.levels))
+        see = (rays & tile_pixels<kW, kH>(view, v.cluster_lo[v.cl.first[top] + lane],
+                                          v.cluster_hi[v.cl.first[top] + lane])) != 0u;
+      const uint32_t m = __ballot_sync(0xffffffffu, see);
+      if (lane == 0) {
+        w.mask[top] = m;
+        w.base[top] = 0u;
+      }
+      __syncwarp();
+    }
+    while (true) {
+      // ---- descend until more than 32 leaves are at hand ----------------
+      while (filled <= 32u && !done) {
+        const uint32_t m = w.mask[lev];
+        const uint32_t node = w.base[lev] + __ffs(m) - 1u;
+        __syncwarp();
+        if (m == 0u) {
+          if (lev == top) done = true;
+          else ++lev;
+          continue;
+        }
+        if (lane == 0) w.mask[lev] = m & (m - 1u);
+        const uint32_t child = node * 32u + lane;
+        if (lev > 0) {
+          --lev;
+          bool see = false;
+          if (child < boxes_above(n, 5u * (uint32_t)(lev + 1)))
+            see = (rays & tile_pixels<kW, kH>(view, v.cluster_lo[v.cl.first[lev] + child],
+                                              v.cluster_hi[v.cl.first[lev] + child])) != 0u;
+          const uint32_t cm = __ballot_sync(0xffffffffu, see);
+          if (lane == 0) {
+            w.mask[lev] = cm;
+            w.base[lev] = node * 32u;
+          }
+        } else {
+          float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+          uint32_t covers = 0u;
+          if (child < n) {
+            lo = v.leaf.lo[child];
+            hi = v.leaf.hi[child];
+            covers = rays & tile_pixels<kW, kH>(view, lo, hi);
+          }
+          const uint32_t cm = __ballot_sync(0xffffffffu, covers != 0u);
+          if (covers) {
+            const float4 A = v.leaf.a[child], B = v.leaf.b[child];
+            const uint32_t beam = v.leaf.beam[child];
+            const f3 ax = mk(B.x, B.y, B.z) - mk(A.x, A.y, A.z);
+            const float segl = length(ax);
+            const uint32_t at = filled + __popc(cm & lt);
+            float4* f = w.leaf[at];
+            f[0] = make_float4(lo.x, lo.y, lo.z, B.w);
+            f[1] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(beam));
+            f[2] = A;
+            f[3] = make_float4(ax.x / segl, ax.y / segl, ax.z / segl, segl);
+            w.pixels[at] = covers;
+          }
+          filled += __popc(cm);
+        }
+        __syncwarp();
+      }
+      if (filled == 0u) break;
+      // ---- the batch's pairs, in leaf order -------------------------------
+      uint32_t qh = 0, qn = 0;
+      for (uint32_t half = 0; half < filled; half += 32u) {
+        uint32_t pm = half + lane < filled ? w.pixels[half + lane] : 0u;
+        uint32_t at = __popc(pm);  // inclusive prefix of the lanes' pair counts
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+          const uint32_t x = __shfl_up_sync(0xffffffffu, at, k);
+          if (lane >= (uint32_t)k) at += x;
+        }
+        const uint32_t pairs = __shfl_sync(0xffffffffu, at, 31);
+        at -= __popc(pm);
+        for (; pm; pm &= pm - 1u) w.pair[at++] = (uint16_t)(((half + lane) << 5) | (__ffs(pm) - 1u));
+        __syncwarp();
+        for (uint32_t i = 0; i < pairs; i += 32u) {
+          bool pass = false;
+          float t = 0.0f, sb = 0.0f;
+          uint32_t id = 0;
+          if (i + lane < pairs) {
+            id = w.pair[i + lane];
+            const float4* f = w.leaf[id >> 5];
+            const float4* q = w.ray[id & 31u];
+            const float4 r0 = q[0], r1 = q[1], r2 = q[2];
+            const f3 o = mk(r0.x, r0.y, r0.z);
+            if (ray_box(o, mk(r2.x, r2.y, r2.z), r0.w, r2.w, f[0], f[1])) {
+              ++segs;
+              const float4 a = f[2], d = f[3];
+              pass = beam_closest(mk(a.x, a.y, a.z), a.w, mk(d.x, d.y, d.z), d.w, o, mk(r1.x, r1.y, r1.z), r0.w, r1.w,
+                                  t, sb);
+            }
+          }
+          const uint32_t acc = __ballot_sync(0xffffffffu, pass);
+          if (pass) {
+            const uint32_t k = (qh + qn + __popc(acc & lt)) & 63u;
+            w.q_id[k] = id;
+            w.q_t[k] = make_float2(t, sb);
+          }
+          qn += __popc(acc);
+          const bool last = i + 32u >= pairs && half + 32u >= filled;  // the leaf slots are refilled after it
+          while (qn >= 32u || (last && qn)) {
+            // ---- a group of up to 32 pairs, one lane each ------------------
+            const uint32_t m = min(qn, 32u);
+            if (lane < (uint32_t)P) w.own[lane] = 0u;
+            __syncwarp();
+            f3 c = mk(0.f, 0.f, 0.f);
+            uint32_t key = 32u + lane;
+            if (lane < m) {
+              const uint32_t k = (qh + lane) & 63u, e = w.q_id[k];
+              const float2 ts = w.q_t[k];
+              key = e & 31u;
+              const float4* f = w.leaf[e >> 5];
+              const float4 a = f[2], d = f[3], r0 = w.ray[key][0], r1 = w.ray[key][1];
+              const uint32_t beam = __float_as_uint(f[1].w);
+              const uint32_t pixel = (ty0 + key / kW) * pv.cw + tx0 + key % kW;
+              c = beam_contribution(g, s, v.slots + (size_t)beam * kSlotFloats, mk(a.x, a.y, a.z), a.w,
+                                    mk(d.x, d.y, d.z), f[0].w, mk(r0.x, r0.y, r0.z), mk(r1.x, r1.y, r1.z), r0.w, ts.x,
+                                    ts.y, v.cam_dist + (size_t)pixel * kBeamDists, lookups);
+            }
+            const uint32_t peers = __match_any_sync(0xffffffffu, key);
+            if (lane < m && (peers & lt) == 0u) w.own[key] = peers;
+            w.c[0][lane] = c.x;
+            w.c[1][lane] = c.y;
+            w.c[2][lane] = c.z;
+            __syncwarp();
+            if (lane < (uint32_t)P)
+              for (uint32_t b = w.own[lane]; b; b &= b - 1u) {
+                const int j = __ffs(b) - 1;
+                L = L + mk(w.c[0][j], w.c[1][j], w.c[2][j]);
+              }
+            __syncwarp();
+            qh += m;
+            qn -= m;
+          }
+        }
+        __syncwarp();
+      }
+      filled = 0;
+      if (done) break;
+    }
+  }
+  if (valid) write_result(pv, sum, (pv.y0 + cy) * pv.width + pv.x0 + cx, L);
+  flush_counters(cnt, valid ? 1ull : 0ull, lookups, 0, 0);
   warp_count(evaluated, segs);
+}
+
+template <int P>
+static vcr_status gather_launch_t(vcr_ctx* ctx, const GridView& g, const SceneView& s, const CamView& cam,
+                                  const PassView& pv, const PpbGatherView& gv, Counters cnt,
+                                  unsigned long long* d_count, cudaStream_t st) {
+  constexpr uint32_t kW = gather_w(P), kH = (uint32_t)P / kW;
+  constexpr size_t smem = kGatherWarps * sizeof(GatherWarp<P>);
+  static_assert(smem <= 48 * 1024, "static shared memory limit");
+  const uint32_t tiles = ((pv.cw + kW - 1u) / kW) * ((pv.ch + kH - 1u) / kH);
+  ppb_gather_kernel<P><<<(tiles + kGatherWarps - 1) / kGatherWarps, kGatherThreads, smem, st>>>(
+      g, s, cam, pv, gv, ctx->d_sum, cnt, d_count);
+  VCR_CUDA(ctx, cudaGetLastError());
+  return VCR_OK;
+}
+
+// The largest tile that still gives the SMs 84 tiles each, three and a half
+// rounds of the 24 warps an SM holds: a larger tile shares a leaf's set-up
+// among more pixels, a smaller one leaves less work to the longest warp.
+// Measured (gather ms at 32 / 16 / 8 / 4 / 2 pixels a tile, 256^3 cloud):
+// 1280x720, 9.6 M segments 29.1 / 29.3 / 36.3 / 49.0 / -; 640x360, 3.1 M
+// segments 4.98 / 4.40 / 4.57 / 5.72 / -; 320x180 5.11 / 3.31 / 2.41 / 2.36 /
+// -; 160x90 6.20 / 3.91 / 2.61 / 1.89 / 1.61.
+static vcr_status gather_launch(vcr_ctx* ctx, const GridView& g, const SceneView& s, const CamView& cam,
+                                const PassView& pv, const PpbGatherView& gv, Counters cnt,
+                                unsigned long long* d_count, cudaStream_t st) {
+  const auto fits = [&](uint32_t w, uint32_t h) {
+    return (uint64_t)((pv.cw + w - 1u) / w) * ((pv.ch + h - 1u) / h) >= 84ull * (uint32_t)ctx->sm_count;
+  };
+  if (fits(8, 4)) return gather_launch_t<32>(ctx, g, s, cam, pv, gv, cnt, d_count, st);
+  if (fits(4, 4)) return gather_launch_t<16>(ctx, g, s, cam, pv, gv, cnt, d_count, st);
+  if (fits(4, 2)) return gather_launch_t<8>(ctx, g, s, cam, pv, gv, cnt, d_count, st);
+  if (fits(2, 2)) return gather_launch_t<4>(ctx, g, s, cam, pv, gv, cnt, d_count, st);
+  return gather_launch_t<2>(ctx, g, s, cam, pv, gv, cnt, d_count, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -527,10 +956,11 @@ __global__ void __launch_bounds__(kGatherThreads) ppb_gather_kernel(GridView g, 
 static void ppb_release(PpbState* st) {
   void* ptrs[] = {st->slots,      st->nbeams,      st->slot_segs,   st->slot_off,   st->photon_segs,
                   st->photon_off, st->scan_sums,   st->total,       st->seg_a,      st->seg_b,
-                  st->leaf_a,     st->leaf_b,      st->leaf_beam,   st->node_pk,    st->seg_beam,
+                  st->leaf_a,     st->leaf_b,      st->leaf_beam,   st->cluster_lo, st->seg_beam,
                   st->codes,      st->idx,         st->codes_sorted, st->idx_sorted, st->left,
                   st->right,      st->parent_int,  st->parent_leaf, st->flags,      st->leaf_lo,
-                  st->leaf_hi,    st->node_lo,     st->node_hi,     st->node2};
+                  st->leaf_hi,    st->node_lo,     st->node_hi,     st->cluster_hi, st->cam_dist,
+                  st->live_lo,    st->live_hi,     st->live_mask,   st->live_off,   st->reach};
   for (void* p : ptrs) cudaFree(p);
   probe_free(st->gather);
 }
@@ -573,8 +1003,13 @@ vcr_status ppb_setup(vcr_ctx* ctx, const vcr_ppb_params* p) {
   VCR_ALLOC(st->total, 4);
   VCR_ALLOC(st->seg_a, C * sizeof(float4));
   VCR_ALLOC(st->seg_b, C * sizeof(float4));
-  VCR_ALLOC(st->node_pk, 2 * C * sizeof(float4));
-  VCR_ALLOC(st->node2, 6 * C * sizeof(float4));
+  VCR_ALLOC(st->live_lo, C * sizeof(float4));
+  VCR_ALLOC(st->live_hi, C * sizeof(float4));
+  VCR_ALLOC(st->live_mask, (C + 31) / 32 * 4);
+  VCR_ALLOC(st->live_off, (C + 31) / 32 * 4);
+  VCR_ALLOC(st->reach, P * K * 4);
+  VCR_ALLOC(st->cluster_lo, cluster_layout((uint32_t)C).total * sizeof(float4));
+  VCR_ALLOC(st->cluster_hi, cluster_layout((uint32_t)C).total * sizeof(float4));
   VCR_ALLOC(st->leaf_a, C * sizeof(float4));
   VCR_ALLOC(st->leaf_b, C * sizeof(float4));
   VCR_ALLOC(st->leaf_beam, C * 4);
@@ -594,15 +1029,6 @@ vcr_status ppb_setup(vcr_ctx* ctx, const vcr_ppb_params* p) {
   VCR_ALLOC(st->node_hi, C * sizeof(float4));
 #undef VCR_ALLOC
   return ensure_scratch(ctx, sort_scratch_bytes(p->capacity));
-}
-
-// node2 (two tree levels per internal node, lbvh_node2_kernel) of a refit tree of n leaves.
-vcr_status lbvh_node2(vcr_ctx* ctx, const float4* node_pk, const float4* leaf_lo, const float4* leaf_hi, int n,
-                      float4* node2, cudaStream_t st) {
-  if (n <= 1) return VCR_OK;
-  lbvh_node2_kernel<<<ctx->sm_count * 8, 256, 0, st>>>(node_pk, leaf_lo, leaf_hi, (uint32_t)(n - 1), node2);
-  VCR_CUDA(ctx, cudaGetLastError());
-  return VCR_OK;
 }
 
 vcr_status lbvh_build_refit(vcr_ctx* ctx, const uint32_t* codes, const uint32_t* order, const float4* seg_a,
@@ -637,7 +1063,7 @@ vcr_status ppb_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
   st->radius = ppb_radius_at(st->prm.radius, st->prm.alpha, pass->pass_index);
   Counters cnt{ctx->d_counters};
   VCR_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0, 5 * sizeof(unsigned long long), st_));
-  PpbEmitView ev{st->slots, st->nbeams, st->slot_segs, st->slot_off, st->photon_segs, P, K, st->radius,
+  PpbEmitView ev{st->slots, st->nbeams, st->slot_segs, st->slot_off, st->photon_segs, st->reach, P, K, st->radius,
                  pass->seed, pass->pass_index};
   ppb_emit_kernel<<<(P + 127) / 128, 128, 0, st_>>>(g, s, ev, cnt);
   VCR_CUDA(ctx, cudaGetLastError());
@@ -657,25 +1083,67 @@ vcr_status ppb_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
                                    st->idx_sorted, n, 0, 30, st_));
   vs = lbvh_build_refit(ctx, st->codes_sorted, st->idx_sorted, st->seg_a, st->seg_b, (int)n, st->left, st->right,
                         st->parent_int, st->parent_leaf, st->flags, st->leaf_lo, st->leaf_hi, st->node_lo,
-                        st->node_hi, st_, st->node_pk);
+                        st->node_hi, st_, nullptr);
   if (vs) return vs;
+  // the gather's leaves and clusters
+  PpbGatherView gv{};
+  gv.cl = cluster_layout(n);
+  gv.leaf = GatherLeaves{st->leaf_a, st->leaf_b, st->live_lo, st->live_hi, st->leaf_beam};
+  gv.n_live = st->total;  // n's copy is on the host by now
   if (n) {
-    ppb_leaf_order_kernel<<<ctx->sm_count * 8, 256, 0, st_>>>(st->idx_sorted, st->seg_a, st->seg_b, st->seg_beam, n,
-                                                              st->leaf_a, st->leaf_b, st->leaf_beam);
+    LiveView lv{st->idx_sorted, st->seg_a, st->seg_b, st->seg_beam, st->reach, nullptr, {0, 0, 0}, s.b0, f3{}};
+    // the finest majorant level whose cells are at least as wide as a
+    // segment's box is thick: the box then spans few of them
+    int level = 0;
+    const f3 ext = s.b1 - s.b0;
+    f3 cell{};
+    for (;; ++level) {
+      const float voxels = (float)(kBrick << level);
+      cell = mk(ext.x / (float)ctx->gdesc.size[0] * voxels, ext.y / (float)ctx->gdesc.size[1] * voxels,
+                ext.z / (float)ctx->gdesc.size[2] * voxels);
+      if (level == 3 || std::min(cell.x, std::min(cell.y, cell.z)) >= 2.0f * st->radius) break;
+    }
+    lv.maj = ctx->d_majorants + ctx->moff[level];
+    for (int a = 0; a < 3; ++a) lv.mnb[a] = ctx->mnb[level][a];
+    lv.icell = mk(1.0f / cell.x, 1.0f / cell.y, 1.0f / cell.z);
+    const uint32_t c = (n + 31u) / 32u;
+    ppb_live_kernel<<<(c + 7u) / 8u, 256, 0, st_>>>(lv, n, st->live_mask, st->flags);
     VCR_CUDA(ctx, cudaGetLastError());
+    VCR_CUDA(ctx, exclusive_scan_u32(st->flags, st->live_off, c, st->scan_sums, st->total, st_));
+    ppb_compact_kernel<<<(c + 7u) / 8u, 256, 0, st_>>>(st->idx_sorted, st->seg_a, st->seg_b, st->seg_beam,
+                                                       st->leaf_lo, st->leaf_hi, n, st->live_mask, st->live_off,
+                                                       gv.leaf);
+    VCR_CUDA(ctx, cudaGetLastError());
+    for (int l = 0; l < gv.cl.levels; ++l) {
+      const float4* lo_in = l ? st->cluster_lo + gv.cl.first[l - 1] : st->live_lo;
+      const float4* hi_in = l ? st->cluster_hi + gv.cl.first[l - 1] : st->live_hi;
+      ppb_cluster_kernel<<<(gv.cl.count[l] + 7u) / 8u, 256, 0, st_>>>(lo_in, hi_in, gv.n_live, 5u * (uint32_t)l,
+                                                                     st->cluster_lo + gv.cl.first[l],
+                                                                     st->cluster_hi + gv.cl.first[l]);
+      VCR_CUDA(ctx, cudaGetLastError());
+    }
   }
-  vs = lbvh_node2(ctx, st->node_pk, st->leaf_lo, st->leaf_hi, (int)n, st->node2, st_);
-  if (vs) return vs;
-  PpbGatherView gv{st->leaf_a,  st->leaf_b, st->leaf_beam, st->slots,      st->leaf_lo,
-                   st->leaf_hi, st->node2, (int)n,        pass->seed, pass->pass_index};
-  // one warp per 8x4 pixel tile
-  uint32_t tiles = ((pv.cw + 7u) / 8u) * ((pv.ch + 3u) / 4u);
-  uint32_t warps_per_block = kGatherThreads / 32;
+  const size_t pixels = (size_t)pv.cw * pv.ch;
+  if (st->cam_pixels < pixels) {  // kept for the next pass; frames may grow after the set-up
+    cudaFree(st->cam_dist);
+    st->cam_dist = nullptr;
+    st->cam_pixels = 0;
+    VCR_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&st->cam_dist), pixels * kBeamDists * sizeof(float)));
+    st->cam_pixels = pixels;
+  }
+  gv.slots = st->slots;
+  gv.radius = st->radius;
+  gv.cluster_lo = st->cluster_lo;
+  gv.cluster_hi = st->cluster_hi;
+  gv.cam_dist = st->cam_dist;
+  gv.seed = pass->seed;
+  gv.pass = pass->pass_index;
   vcr_status ps = probe_begin(ctx, st->gather, st_);
   if (ps) return ps;
-  ppb_gather_kernel<<<(tiles + warps_per_block - 1) / warps_per_block, kGatherThreads, 0, st_>>>(
-      g, s, cam_view(ctx->cam), pv, gv, ctx->d_sum, cnt, st->gather.d_count);
+  ppb_camera_kernel<<<(unsigned)((pixels + 127) / 128), 128, 0, st_>>>(g, s, cam_view(ctx->cam), pv, gv, cnt);
   VCR_CUDA(ctx, cudaGetLastError());
+  vs = gather_launch(ctx, g, s, cam_view(ctx->cam), pv, gv, cnt, st->gather.d_count, st_);
+  if (vs) return vs;
   ps = probe_end(ctx, st->gather, st_);
   if (ps) return ps;
   VCR_CUDA(ctx, cudaEventRecord(ctx->work_done, st_));

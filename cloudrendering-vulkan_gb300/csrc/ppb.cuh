@@ -14,7 +14,7 @@ constexpr int kSlotFloats = 28;            // start 3, dir 3, length, power 3, 1
 constexpr uint32_t kMaxBeamsPerPhoton = 65;  // 64 scatter events + the entering beam
 constexpr uint32_t kMaxSegPerBeam = 4096;
 constexpr uint32_t kLeafBit = 0x80000000u;
-constexpr int kGatherStack = 64;
+constexpr int kGatherStack = 64;  // tree walks over packed nodes
 constexpr uint32_t kEmitSalt = 0x85EBCA6Bu;
 constexpr uint32_t kGatherSalt = 0xC2B2AE35u;
 
@@ -27,15 +27,18 @@ struct PpbState {
   uint32_t *nbeams = nullptr, *slot_segs = nullptr, *slot_off = nullptr, *photon_segs = nullptr,
            *photon_off = nullptr, *scan_sums = nullptr, *total = nullptr;
   float4 *seg_a = nullptr, *seg_b = nullptr;
-  // the segments again in the LBVH's leaf (Morton) order, for the gather:
-  // leaf i's segment is at i, loaded together with the leaf's box
-  float4 *leaf_a = nullptr, *leaf_b = nullptr;
-  uint32_t* leaf_beam = nullptr;
+  // the segments that can contribute, with their boxes, in the LBVH's leaf
+  // (Morton) order, for the gather
+  float4 *leaf_a = nullptr, *leaf_b = nullptr, *live_lo = nullptr, *live_hi = nullptr;
+  uint32_t *leaf_beam = nullptr, *live_mask = nullptr, *live_off = nullptr;  // the latter two per 32 leaves
+  float* reach = nullptr;  // per beam slot: the farthest of its transmittance distances
   uint32_t *seg_beam = nullptr, *codes = nullptr, *idx = nullptr, *codes_sorted = nullptr, *idx_sorted = nullptr;
   uint32_t *left = nullptr, *right = nullptr, *parent_int = nullptr, *parent_leaf = nullptr, *flags = nullptr;
   float4 *leaf_lo = nullptr, *leaf_hi = nullptr, *node_lo = nullptr, *node_hi = nullptr;
-  float4* node_pk = nullptr;  // internal nodes packed for the gather: (lo, left), (hi, right)
-  float4* node2 = nullptr;    // per internal node: its packed node and its two children's (6 float4)
+  // the gather's clusters: boxes over 32 consecutive of those, over 32 of these, ...
+  float4 *cluster_lo = nullptr, *cluster_hi = nullptr;
+  float* cam_dist = nullptr;  // per pixel of a pass: the 16 free flights along the camera ray, ascending
+  size_t cam_pixels = 0;
   GatherProbe gather;  // segments the last gather evaluated, its device time
 };
 
