@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(128) ppb_camera_kernel(GridView g, SceneView s
         float tau = -vlog(rng_next(rng));
         bool ended = true;
         float t = kEscaped;
-        if (track_walk(tr, g, g.majorants, s.k_sigma, tau, cells, 0xFFFFFFFFu) == kCandidate) {
+        if (track_walk(tr, g.majorants, s.k_sigma, tau, cells, 0xFFFFFFFFu) == kCandidate) {
           const float rho = density_at(g, s, along(entry, rd, tr.t));
           ++lookups;
           if (rng_next(rng) * tr.m < rho) t = tr.t;

@@ -179,17 +179,12 @@ struct Dda {
 // once per ray and shared with the slab test) and by the reciprocal cell
 // size `ics`, so a ray's DDA costs three divisions in all; the sign test is
 // on d itself because 1/(+-0) is +-inf.
+// (Selects instead of branches: neighbouring lanes' rays point everywhere.)
 VCR_HD void dda_axis_init(float o, float d, float inv, float b0, float cs, int c, float& tmax, float& tdel) {
-  if (d > 0.0f) {
-    tmax = ((b0 + (float)(c + 1) * cs) - o) * inv;
-    tdel = cs * inv;
-  } else if (d < 0.0f) {
-    tmax = ((b0 + (float)c * cs) - o) * inv;
-    tdel = cs * inv;  // negative: the axis steps down
-  } else {
-    tmax = INFINITY;
-    tdel = INFINITY;
-  }
+  const bool moves = d > 0.0f || d < 0.0f;
+  const float edge = b0 + (float)(d > 0.0f ? c + 1 : c) * cs;
+  tmax = moves ? (edge - o) * inv : INFINITY;
+  tdel = moves ? cs * inv : INFINITY;  // negative: the axis steps down
 }
 
 VCR_HD int cell_of(float o, float b0, float ics, int nc) {
@@ -210,36 +205,25 @@ VCR_HD float dda_cell_exit(const Dda& d) { return fminf(fminf(d.tmax[0], d.tmax[
 
 // Advance to the next cell; false when it leaves the grid.  The step is the
 // sign of tdel and tmax grows by |tdel| (the cell's t extent).
-// (Each axis is spelled out so the state stays in registers.)
+// (Each axis is spelled out so the state stays in registers, and selected
+// rather than branched to: the lanes of a warp cross different faces.)
+VCR_HD int dda_step_of(float tdel) { return tdel < 0.0f ? -1 : 1; }
 VCR_HD bool dda_advance(Dda& d, const int nc[3]) {
-  if (d.tmax[0] <= d.tmax[1] && d.tmax[0] <= d.tmax[2]) {
-    d.c[0] += d.tdel[0] < 0.0f ? -1 : 1;
-    d.tmax[0] = d.tmax[0] + fabsf(d.tdel[0]);
-    return d.c[0] >= 0 && d.c[0] < nc[0];
-  }
-  if (d.tmax[1] <= d.tmax[2]) {
-    d.c[1] += d.tdel[1] < 0.0f ? -1 : 1;
-    d.tmax[1] = d.tmax[1] + fabsf(d.tdel[1]);
-    return d.c[1] >= 0 && d.c[1] < nc[1];
-  }
-  d.c[2] += d.tdel[2] < 0.0f ? -1 : 1;
-  d.tmax[2] = d.tmax[2] + fabsf(d.tdel[2]);
-  return d.c[2] >= 0 && d.c[2] < nc[2];
+  const bool x = d.tmax[0] <= d.tmax[1] && d.tmax[0] <= d.tmax[2];
+  const bool y = !x && d.tmax[1] <= d.tmax[2];
+  const bool z = !x && !y;
+  d.c[0] += x ? dda_step_of(d.tdel[0]) : 0;
+  d.c[1] += y ? dda_step_of(d.tdel[1]) : 0;
+  d.c[2] += z ? dda_step_of(d.tdel[2]) : 0;
+  d.tmax[0] = x ? d.tmax[0] + fabsf(d.tdel[0]) : d.tmax[0];
+  d.tmax[1] = y ? d.tmax[1] + fabsf(d.tdel[1]) : d.tmax[1];
+  d.tmax[2] = z ? d.tmax[2] + fabsf(d.tdel[2]) : d.tmax[2];
+  return (uint32_t)d.c[0] < (uint32_t)nc[0] && (uint32_t)d.c[1] < (uint32_t)nc[1] &&
+         (uint32_t)d.c[2] < (uint32_t)nc[2];
 }
 
 VCR_HD uint32_t dda_linear(const Dda& d, const int nc[3]) {
   return (uint32_t)d.c[0] + (uint32_t)nc[0] * ((uint32_t)d.c[1] + (uint32_t)nc[1] * (uint32_t)d.c[2]);
 }
-
-// One free-flight sample against piecewise-constant majorants: consume the
-// optical depth tau = -ln(u) cell by cell.  Returns true with t at a
-// tentative collision inside the current cell (majorant *m, density units),
-// false when the segment [t, t_end] is used up.
-//   per cell: e = min(tmax), s = min(e, t_end), dtau = (m*k)*(s - t);
-//   if dtau > tau: t = t + tau/(m*k), stop; else tau -= dtau, t = s, advance.
-struct TrackState {
-  Dda dda;
-  float t, t_end, m;
-};
 
 }  // namespace vcr
