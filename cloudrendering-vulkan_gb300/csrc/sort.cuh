@@ -8,7 +8,7 @@
 
 namespace vcr {
 
-constexpr uint32_t kSortTileKeys = 4096;  // keys per tile (256 threads x 16)
+constexpr uint32_t kSortTileKeys = 4096;  // keys of the smallest tile
 constexpr int kSortDigitBits = 8;         // bits a digit pass sorts on
 constexpr int kSortRadix = 1 << kSortDigitBits;
 constexpr int kSortMaxPasses = 32 / kSortDigitBits;
