@@ -214,6 +214,14 @@ __device__ __forceinline__ bool roulette_survives(Rng& rng, float p, float& beta
 constexpr int kThreadsPerSm = 768;
 // Lanes without a ray before new ones are set up: 6 to 16 measured within 3 %.
 constexpr uint32_t kRefillAt = 10;
+// Training paths run to their end (64 events) where camera paths of the
+// cached tracker end at their second event: each is a chain of dependent
+// steps, and the longest decides when the launch ends.  They start in warps
+// of their own, few a warp, which take camera paths only when theirs are
+// done, so that a step of theirs is short and nothing waits for 32 others.
+// 45 k of them with 4.1 M camera paths: 1,213 us a frame with mixed warps,
+// 976 at 8 to 32 a warp, 1,020 at 96.
+constexpr uint32_t kTrainPerWarp = 16;
 // The paths a warp holds, in shared memory: the lanes fly 32 of them at a
 // time, the others wait in one of the queues.  With 80 the parts ran at 15
 // to 19 lanes and the passes above took 3 % longer; 128 leave two CTAs an SM.
@@ -278,7 +286,7 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
     pt_wavefront_kernel(const __grid_constant__ GridView g, const __grid_constant__ SceneView s,
                         const __grid_constant__ CamView cam, const __grid_constant__ PassView pv,
                         double* __restrict__ sum, uint32_t* __restrict__ stats, Counters cnt, uint32_t total,
-                        uint32_t dda_steps, uint32_t cap, uint32_t maj_bytes,
+                        uint32_t dda_steps, uint32_t cap, uint32_t train_warps, uint32_t maj_bytes,
                         uint32_t stage_polls, const __grid_constant__ NrcSink nq,
                         const __grid_constant__ NrcTrainSink ts, const __grid_constant__ BatchSink bt,
                         int* __restrict__ err) {
@@ -311,6 +319,7 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
   const uint32_t slots = cap < 32u ? cap : (uint32_t)kPool;
   uint32_t n_free = slots, n_done = 0, n_ready = 0, h_ready = 0, n_shade = 0, h_shade = 0;
   bool exhausted = false;
+  bool serving = (threadIdx.x >> 5) * gridDim.x + blockIdx.x < train_warps;
   for (uint32_t i = lane; i < (uint32_t)kPool; i += 32u) pool.free_[i] = (uint8_t)i;
   if (lane < 4u) pool.totals[lane] = 0ull;
   __syncwarp();
@@ -325,7 +334,10 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
 
   while (true) {
     const uint32_t flying = __ballot_sync(0xffffffffu, mode == kFly);
-    if (flying == 0u || 32u - __popc(flying) >= (exhausted ? 1u : kRefillAt)) {
+    // (with no new paths to come only what waits is worth a look, at once)
+    const bool look = exhausted ? n_ready + n_shade != 0u || n_done >= 32u || __any_sync(0xffffffffu, mode == kAim)
+                                : 32u - __popc(flying) >= kRefillAt;
+    if (flying == 0u || look) {
       // ---- hand the lanes without a path one that waits -------------------
       const uint32_t idle = __ballot_sync(0xffffffffu, mode == kIdle);
       const uint32_t n_idle = __popc(idle);
@@ -410,12 +422,13 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
           // ---- new paths ----------------------------------------------------
           const uint32_t take = min(min(n_free, cap), 32u);
           uint32_t base = 0;
-          if (lane == 0) base = (uint32_t)atomicAdd(cnt.c + 4, (unsigned long long)take);
-          base = __shfl_sync(0xffffffffu, base, 0);
-          exhausted = base + take >= total + ts.paths;
+          if (lane == 0) base = (uint32_t)atomicAdd(cnt.c + (serving ? 6 : 4), (unsigned long long)take);
+          base = __shfl_sync(0xffffffffu, base, 0) + (serving || !train_warps ? 0u : ts.paths);
+          const uint32_t end = serving ? ts.paths : total + ts.paths;
+          exhausted = base + take >= end;
           uint32_t id = base + lane, pid = 0, pix = 0;
           bool hit = false;
-          const bool fresh = lane < take && id < total + ts.paths;
+          const bool fresh = lane < take && id < end;
           Rng rng{0u, 0u};
           PathStart ps;
           if (fresh) {
@@ -519,7 +532,11 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
       __syncwarp();
       if (!__any_sync(0xffffffffu, mode == kFly)) {
         // nothing waits either unless it is finished paths
-        if (n_done == 0u) break;
+        if (n_done == 0u) {
+          if (!serving) break;
+          serving = false;  // its training paths are done: camera paths from now on
+          exhausted = total == 0u;
+        }
         continue;
       }
     }
@@ -632,9 +649,10 @@ static vcr_status launch_t(vcr_ctx* ctx, const GridView& g, const SceneView& s, 
   // with one path runs only that path's parts (64x64 pixels: 166 -> 126 us)
   uint32_t cap = (uint32_t)std::min<uint64_t>((paths + (uint64_t)blocks * kWarps - 1) / ((uint64_t)blocks * kWarps), 32u);
   blocks = std::min<uint32_t>(blocks, (uint32_t)((paths + (uint64_t)cap * kWarps - 1) / ((uint64_t)cap * kWarps)));
+  const uint32_t train_warps = cap == 32u && total ? (ts.paths + kTrainPerWarp - 1u) / kTrainPerWarp : 0u;
   NrcSink nq{nullptr, nullptr, 0u};
   if (s.nrc_events && ctx->nrc) nq = NrcSink{ctx->nrc->query, ctx->nrc->query_count, ctx->nrc->query_capacity};
-  kern<<<blocks, kThreads, smem, st>>>(g, s, cam, pv, sum, stats, cnt, total, ctx->tuning.dda_steps, cap, maj_bytes,
+  kern<<<blocks, kThreads, smem, st>>>(g, s, cam, pv, sum, stats, cnt, total, ctx->tuning.dda_steps, cap, train_warps, maj_bytes,
                                        wait_limits().stage_wait, nq, ts, bt, ctx->d_error);
   VCR_CUDA(ctx, cudaGetLastError());
   return VCR_OK;

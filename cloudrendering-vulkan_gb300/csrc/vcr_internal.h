@@ -68,7 +68,7 @@ struct vcr_ctx {
   } rb;
 
   // device counters: [0] paths [1] lookups [2] events [3] dda cells [4] work cursor
-  // [5] grid max (u32 bits) [7] relRMSE accumulator (double bits)
+  // [5] grid max (u32 bits) [6] training-path cursor [7] relRMSE accumulator (double bits)
   unsigned long long* d_counters = nullptr;
   int* d_error = nullptr;  // device error word (bounded waits, index checks)
 
