@@ -1031,16 +1031,22 @@ vcr_status ppb_setup(vcr_ctx* ctx, const vcr_ppb_params* p) {
   return ensure_scratch(ctx, sort_scratch_bytes(p->capacity));
 }
 
+vcr_status lbvh_build(vcr_ctx* ctx, const uint32_t* codes, int n, uint32_t* left, uint32_t* right,
+                      uint32_t* parent_int, uint32_t* parent_leaf, cudaStream_t st) {
+  if (n <= 1) return VCR_OK;
+  lbvh_build_kernel<<<(n - 1 + 255) / 256, 256, 0, st>>>(codes, n, left, right, parent_int, parent_leaf);
+  VCR_CUDA(ctx, cudaGetLastError());
+  return VCR_OK;
+}
+
 vcr_status lbvh_build_refit(vcr_ctx* ctx, const uint32_t* codes, const uint32_t* order, const float4* seg_a,
                             const float4* seg_b, int n, uint32_t* left, uint32_t* right, uint32_t* parent_int,
                             uint32_t* parent_leaf, uint32_t* flags, float4* leaf_lo, float4* leaf_hi,
                             float4* node_lo, float4* node_hi, cudaStream_t st, float4* node_pk) {
   if (n <= 0) return VCR_OK;
-  if (n > 1) {
-    lbvh_build_kernel<<<(n - 1 + 255) / 256, 256, 0, st>>>(codes, n, left, right, parent_int, parent_leaf);
-    VCR_CUDA(ctx, cudaGetLastError());
-    VCR_CUDA(ctx, cudaMemsetAsync(flags, 0, (size_t)(n - 1) * 4, st));
-  }
+  vcr_status vs = lbvh_build(ctx, codes, n, left, right, parent_int, parent_leaf, st);
+  if (vs) return vs;
+  if (n > 1) VCR_CUDA(ctx, cudaMemsetAsync(flags, 0, (size_t)(n - 1) * 4, st));
   lbvh_refit_kernel<<<(n + 255) / 256, 256, 0, st>>>(seg_a, seg_b, order, n, left, right, parent_int, parent_leaf,
                                                      flags, leaf_lo, leaf_hi, node_lo, node_hi, node_pk);
   VCR_CUDA(ctx, cudaGetLastError());

@@ -30,6 +30,8 @@
 
 namespace vcr {
 
+vcr_status lbvh_build(vcr_ctx* ctx, const uint32_t* codes, int n, uint32_t* left, uint32_t* right,
+                      uint32_t* parent_int, uint32_t* parent_leaf, cudaStream_t st);
 vcr_status lbvh_build_refit(vcr_ctx* ctx, const uint32_t* codes, const uint32_t* order, const float4* seg_a,
                             const float4* seg_b, int n, uint32_t* left, uint32_t* right, uint32_t* parent_int,
                             uint32_t* parent_leaf, uint32_t* flags, float4* leaf_lo, float4* leaf_hi,
@@ -172,7 +174,7 @@ __host__ __device__ __forceinline__ double ppm_cbrt_ratio(double r) {
 }
 
 // Photon powers and directions in the tree's leaf order: leaf i holds
-// photon order[i].
+// photon order[i] (the march, which visits every leaf's photon).
 __global__ void ppm_leaf_order_kernel(const uint32_t* __restrict__ order, const float4* __restrict__ pw,
                                       const float4* __restrict__ dir, uint32_t n, float4* __restrict__ leaf_pw,
                                       float4* __restrict__ leaf_dir) {
@@ -183,15 +185,103 @@ __global__ void ppm_leaf_order_kernel(const uint32_t* __restrict__ order, const 
   }
 }
 
-// What the gather and the march read: photon powers and directions in the
-// tree's leaf order (leaf i holds photon order[i]), the leaf positions, and
-// the internal nodes packed as (low corner, left child bits) (high corner,
-// right child bits).
+// Boxes over 8 consecutive photons of the leaf order (level 0), over 8 of
+// those (level 1), ... up to the first level of at most 8; box i of a level
+// at box[2 (first + i)] (low corner) and the next (high corner).
+constexpr int kOctLevels = 10;  // 8^10 = 2^30 > 2^28 photons
+struct OctLayout {
+  uint32_t first[kOctLevels];  // the level's first box
+  uint32_t count[kOctLevels];
+  uint32_t total;
+  int levels;
+};
+static OctLayout oct_layout(uint32_t photons) {
+  OctLayout o{};
+  uint32_t n = photons;
+  do {
+    n = (n + 7u) / 8u;
+    o.count[o.levels] = n;
+    o.first[o.levels++] = o.total;
+    o.total += n;
+  } while (n > 8u && o.levels < kOctLevels);
+  return o;
+}
+
+// Three levels at a time, from the level `below` (its boxes, or the photons
+// in their order, whose positions the first call also copies): a CTA's 512
+// inputs make 64 boxes, 8 of the next level and one of the third.
+constexpr int kOctThreads = 512;
+__device__ __forceinline__ void oct_union(float4& lo, float4& hi) {  // of 8 neighbouring lanes
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
+    lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
+    lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
+    hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
+    hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
+    hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
+  }
+}
+__global__ void __launch_bounds__(kOctThreads) oct_kernel(const uint32_t* __restrict__ order,
+                                                          const float4* __restrict__ pos,
+                                                          float4* __restrict__ leaf_pos, float4* __restrict__ box,
+                                                          OctLayout ol, int level, uint32_t n) {
+  __shared__ float4 s_lo[kOctThreads / 8], s_hi[kOctThreads / 8];
+  uint32_t i = blockIdx.x * kOctThreads + threadIdx.x;
+  const float4 none_lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
+  const float4 none_hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+  float4 lo = none_lo, hi = none_hi;
+  if (i < n) {
+    if (level == 0) {
+      lo = hi = pos[order[i]];
+      leaf_pos[i] = lo;
+    } else {
+      const float4* b = box + 2 * (size_t)(ol.first[level - 1] + i);
+      lo = b[0];
+      hi = b[1];
+    }
+  }
+  uint32_t t = threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {  // inputs of step k: threads t < 512 / 8^k
+    oct_union(lo, hi);
+    n = (n + 7u) / 8u;
+    i >>= 3;
+    const uint32_t width = kOctThreads >> (3 * k);
+    if (t < width && (t & 7u) == 0u) {
+      if (level + k < ol.levels && i < n) {
+        float4* b = box + 2 * (size_t)(ol.first[level + k] + i);
+        b[0] = lo;
+        b[1] = hi;
+      }
+      s_lo[t >> 3] = lo;
+      s_hi[t >> 3] = hi;
+    }
+    __syncthreads();
+    lo = t < width / 8u ? s_lo[t] : none_lo;
+    hi = t < width / 8u ? s_hi[t] : none_hi;
+    i = (blockIdx.x * kOctThreads >> (3 * (k + 1))) + t;
+    __syncthreads();
+  }
+}
+
+// What the march reads: photon powers and directions in the tree's leaf
+// order (leaf i holds photon order[i]), the leaf positions, and the internal
+// nodes packed as (low corner, left child bits) (high corner, right child
+// bits).  The gather: the leaf positions, the boxes of 8 above them, and the
+// photons by their order.
 struct PpmGatherView {
   const float4* pw;
   const float4* dir;
   const float4* leaf_lo;
   const float4* node_pk;
+  const uint32_t* order;
+  const float4* box;
+  OctLayout ol;
+  // pixels with a measurement point: their number, the points with sigma_t, the pixels
+  uint32_t* points;
+  float4* point;
+  uint32_t* point_pix;
   int n;
   double* stats;  // per pixel: N, R, tau rgb, background rgb
   float alpha;
@@ -205,20 +295,58 @@ __device__ __forceinline__ float box_dist2(f3 x, float4 lo, float4 hi) {
   return (dx * dx + dy * dy) + dz * dz;
 }
 
-__global__ void __launch_bounds__(128, 8) ppm_gather_kernel(GridView g, SceneView s, CamView cam, PassView pv,
-                                                         PpmGatherView v, double* __restrict__ sum, Counters cnt,
-                                                         unsigned long long* __restrict__ tested) {
-  uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t lookups = 0, cells = 0, found = 0, cand = 0;
-  if (id < pv.cw * pv.ch) {
-    uint32_t cy = id / pv.cw, cx = id - cy * pv.cw;
-    int x = (int)(pv.x0 + cx), y = (int)(pv.y0 + cy);
-    uint32_t pix = (uint32_t)y * pv.width + (uint32_t)x;
-    double* st = v.stats + 8 * (size_t)pix;
-    f3 o, rd;
+// The progressive update of a pixel (FP64): M photons of summed contribution
+// phi, background bg of the pass; then the current estimate, expressed as a
+// sum over the passes so far.
+__device__ __forceinline__ void ppm_update(const PpmGatherView& v, const SceneView& s, uint32_t pix, uint32_t M, f3 phi,
+                                           f3 bg, double* __restrict__ sum) {
+  double* st = v.stats + 8 * (size_t)pix;
+  double N = st[0], R = st[1];
+  double tau[3] = {st[2], st[3], st[4]};
+  if (M > 0) {
+    double am = (double)v.alpha * (double)M;
+    double ratio = (N + am) / (N + (double)M);
+    st[0] = N + am;
+    st[1] = R * ppm_cbrt_ratio(ratio);
+    tau[0] = (tau[0] + (double)phi.x) * ratio;
+    tau[1] = (tau[1] + (double)phi.y) * ratio;
+    tau[2] = (tau[2] + (double)phi.z) * ratio;
+    st[2] = tau[0];
+    st[3] = tau[1];
+    st[4] = tau[2];
+  }
+  st[5] += (double)bg.x;
+  st[6] += (double)bg.y;
+  st[7] += (double)bg.z;
+  double Rn = st[1];
+  double vol = (4.0 / 3.0) * 3.14159265358979323846 * Rn * Rn * Rn;
+  double a = (double)s.albedo / vol;
+  double* o3 = sum + 3 * (size_t)pix;
+  o3[0] = st[5] + a * tau[0];
+  o3[1] = st[6] + a * tau[1];
+  o3[2] = st[7] + a * tau[2];
+}
+
+// One thread a pixel: the camera ray's collision.  Pixels that have one leave
+// their measurement point (with its sigma_t) in a list for the gather, the
+// others are done.
+__global__ void __launch_bounds__(128) ppm_camera_kernel(const __grid_constant__ GridView g,
+                                                         const __grid_constant__ SceneView s,
+                                                         const __grid_constant__ CamView cam,
+                                                         const __grid_constant__ PassView pv,
+                                                         const __grid_constant__ PpmGatherView v,
+                                                         double* __restrict__ sum, Counters cnt) {
+  const uint32_t lane = threadIdx.x & 31u, id = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool in = id < pv.cw * pv.ch;
+  uint32_t lookups = 0, cells = 0, pix = 0;
+  float4 point = make_float4(0.f, 0.f, 0.f, 0.f);
+  bool query = false;
+  if (in) {
+    const uint32_t cy = id / pv.cw, cx = id - cy * pv.cw;
+    const int x = (int)(pv.x0 + cx), y = (int)(pv.y0 + cy);
+    pix = (uint32_t)y * pv.width + (uint32_t)x;
+    f3 o, rd, bg = mk(0.f, 0.f, 0.f);
     camera_ray(cam, x, y, o, rd);
-    f3 bg = mk(0.f, 0.f, 0.f), phi = bg;
-    uint32_t M = 0;
     float tmin, tmax;
     if (!slab(o, rd, s.b0, s.b1, tmin, tmax) || tmax < 0.0f || !(s.ds > 0.0f)) {
       bg = sky(s, rd);
@@ -229,71 +357,190 @@ __global__ void __launch_bounds__(128, 8) ppm_gather_kernel(GridView g, SceneVie
       if (!free_flight(g, s, entry, rd, rng, t, lookups, cells)) {
         bg = sky(s, rd);
       } else if (v.n > 0) {
-        f3 xm = along(entry, rd, t);
-        float sigma_t = s.k_sigma * density_at(g, s, xm);
+        const f3 xm = along(entry, rd, t);
+        point = make_float4(xm.x, xm.y, xm.z, s.k_sigma * density_at(g, s, xm));
         ++lookups;
-        float r = (float)st[1];
-        float r2 = r * r;
-        f3 wo = -rd;
-        uint32_t stack[kGatherStack];
-        int sp = 0;
-        uint32_t node = v.n == 1 ? kLeafBit : 0u;
-        while (true) {
-          if (node & kLeafBit) {
-            uint32_t lf = node & ~kLeafBit;
-            ++cand;
-            float4 q = v.leaf_lo[lf];
-            f3 dq = mk(q.x, q.y, q.z) - xm;
-            if (dot(dq, dq) <= r2) {
-              float4 w = v.dir[lf], pw = v.pw[lf];
-              float f = hg_pdf(s.ph, dot(mk(w.x, w.y, w.z), wo));
-              phi = phi + mk(pw.x, pw.y, pw.z) * f;
-              ++M;
-            }
-          } else {
-            const float4 lo = v.node_pk[2 * (size_t)node], hi = v.node_pk[2 * (size_t)node + 1];
-            if (box_dist2(xm, lo, hi) <= r2) {
-              if (sp < kGatherStack) stack[sp++] = __float_as_uint(hi.w);
-              node = __float_as_uint(lo.w);
-              continue;
-            }
-          }
-          if (sp == 0) break;
-          node = stack[--sp];
-        }
-        if (sigma_t > 0.0f) phi = mk(phi.x / sigma_t, phi.y / sigma_t, phi.z / sigma_t);
-        else phi = mk(0.f, 0.f, 0.f);
+        query = true;
       }
     }
-    // progressive update (FP64)
-    double N = st[0], R = st[1];
-    double tau[3] = {st[2], st[3], st[4]};
-    if (M > 0) {
-      double am = (double)v.alpha * (double)M;
-      double ratio = (N + am) / (N + (double)M);
-      st[0] = N + am;
-      st[1] = R * ppm_cbrt_ratio(ratio);
-      tau[0] = (tau[0] + (double)phi.x) * ratio;
-      tau[1] = (tau[1] + (double)phi.y) * ratio;
-      tau[2] = (tau[2] + (double)phi.z) * ratio;
-      st[2] = tau[0];
-      st[3] = tau[1];
-      st[4] = tau[2];
-    }
-    st[5] += (double)bg.x;
-    st[6] += (double)bg.y;
-    st[7] += (double)bg.z;
-    // current estimate, expressed as a sum over the passes so far
-    double Rn = st[1];
-    double vol = (4.0 / 3.0) * 3.14159265358979323846 * Rn * Rn * Rn;
-    double a = (double)s.albedo / vol;
-    double* o3 = sum + 3 * (size_t)pix;
-    o3[0] = st[5] + a * tau[0];
-    o3[1] = st[6] + a * tau[1];
-    o3[2] = st[7] + a * tau[2];
-    found = M;
+    if (!query) ppm_update(v, s, pix, 0u, mk(0.f, 0.f, 0.f), bg, sum);
   }
-  flush_counters(cnt, id < pv.cw * pv.ch ? 1ull : 0ull, lookups, found, cells);
+  const uint32_t m = __ballot_sync(0xffffffffu, query);
+  uint32_t base = 0;
+  if (m && lane == 0) base = atomicAdd(v.points, (uint32_t)__popc(m));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (query) {
+    const uint32_t at = base + __popc(m & ((1u << lane) - 1u));
+    v.point[at] = point;
+    v.point_pix[at] = pix;
+  }
+  flush_counters(cnt, in ? 1ull : 0ull, lookups, 0, cells);
+}
+
+// What a warp of the gather shares: its measurement points, the boxes of each
+// level still to open, and the photons found but not yet evaluated.
+constexpr uint32_t kPpmChunk = 8;  // measurement points a warp takes at a time
+struct PpmWarp {
+  float4 x[kPpmChunk];            // measurement point, radius^2
+  float4 wo[kPpmChunk];           // direction toward the camera
+  uint32_t open[kOctLevels][32];  // per level: boxes the sphere meets, in order
+  uint8_t next[kOctLevels], count[kOctLevels];
+  uint32_t leaf[64];              // ring of found photons (their leaves), and whose they are
+  uint8_t of[64];
+  float c[3][32];                 // contributions of a group of them
+  uint32_t own[kPpmChunk];        // each point's photons in the group
+};
+
+// The photons within the radius of each measurement point.  A warp takes
+// eight points from the list and looks them up one after the other: a round
+// opens the next four boxes of a level and tests their 32 children (boxes or
+// photons), one lane each; those that the sphere meets, in order, are opened
+// before the level's other boxes.  A photon within the radius lies in boxes
+// within the radius, so the boxes do not change what is found.  The photons
+// found are evaluated (phase toward the camera times power) 32 at a time,
+// whichever points they belong to, and a lane adds its point's in leaf order:
+// the same floats as a walk that visits the leaves in order.
+constexpr int kPpmGatherThreads = 128;
+
+__global__ void __launch_bounds__(kPpmGatherThreads, 8)
+    ppm_gather_kernel(const __grid_constant__ SceneView s, const __grid_constant__ CamView cam,
+                      const __grid_constant__ PassView pv, const __grid_constant__ PpmGatherView v,
+                      double* __restrict__ sum, Counters cnt, unsigned long long* __restrict__ tested) {
+  __shared__ PpmWarp s_w[kPpmGatherThreads / 32];
+  PpmWarp& w = s_w[threadIdx.x >> 5];
+  const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u, slot = lane >> 3, oct = lane & 7u;
+  const uint32_t n = (uint32_t)v.n, points = *v.points;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  const int top = v.ol.levels - 1;
+  uint32_t found_total = 0, cand = 0;
+  for (uint32_t chunk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; chunk * kPpmChunk < points; chunk += warps) {
+    const uint32_t here = min(kPpmChunk, points - chunk * kPpmChunk);
+    uint32_t pix = 0, M = 0;
+    float sigma_t = 0.0f;
+    f3 phi = mk(0.f, 0.f, 0.f);
+    if (lane < here) {
+      const float4 p = v.point[chunk * kPpmChunk + lane];
+      pix = v.point_pix[chunk * kPpmChunk + lane];
+      sigma_t = p.w;
+      const float r = (float)v.stats[8 * (size_t)pix + 1];
+      f3 o, rd;
+      camera_ray(cam, (int)(pix % pv.width), (int)(pix / pv.width), o, rd);
+      w.x[lane] = make_float4(p.x, p.y, p.z, r * r);
+      w.wo[lane] = make_float4(-rd.x, -rd.y, -rd.z, 0.f);
+    }
+    __syncwarp();
+    uint32_t qh = 0, qn = 0;  // the ring's head and count, warp-uniform
+    const auto evaluate = [&]() {  // a group of up to 32 photons, one lane each
+      const uint32_t m = min(qn, 32u);
+      if (lane < kPpmChunk) w.own[lane] = 0u;
+      __syncwarp();
+      f3 c = mk(0.f, 0.f, 0.f);
+      uint32_t key = 32u + lane;
+      if (lane < m) {
+        const uint32_t at = (qh + lane) & 63u, ph = v.order[w.leaf[at]];
+        key = w.of[at];
+        const float4 d = v.dir[ph], pw = v.pw[ph], wo = w.wo[key];
+        c = mk(pw.x, pw.y, pw.z) * hg_pdf(s.ph, dot(mk(d.x, d.y, d.z), mk(wo.x, wo.y, wo.z)));
+      }
+      const uint32_t peers = __match_any_sync(0xffffffffu, key);
+      if (lane < m && (peers & lt) == 0u) w.own[key] = peers;
+      w.c[0][lane] = c.x;
+      w.c[1][lane] = c.y;
+      w.c[2][lane] = c.z;
+      __syncwarp();
+      if (lane < kPpmChunk)
+        for (uint32_t b = w.own[lane]; b; b &= b - 1u) {
+          const int j = __ffs(b) - 1;
+          phi = phi + mk(w.c[0][j], w.c[1][j], w.c[2][j]);
+        }
+      __syncwarp();
+      qh += m;
+      qn -= m;
+    };
+    for (uint32_t j = 0; j < here; ++j) {
+      const float4 q = w.x[j];
+      const f3 x = mk(q.x, q.y, q.z);
+      // the top level's boxes (at most 8)
+      int lev = top;
+      uint32_t next = 0, count = 0;  // of the current level's open boxes
+      {
+        bool hit = false;
+        if (lane < v.ol.count[top]) {
+          const float4* b = v.box + 2 * (size_t)(v.ol.first[top] + lane);
+          hit = box_dist2(x, b[0], b[1]) <= q.w;
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, hit);
+        if (hit) w.open[top][__popc(m & lt)] = lane;
+        count = __popc(m);
+        __syncwarp();
+      }
+      while (true) {
+        if (next >= count) {
+          if (lev == top) break;
+          ++lev;
+          next = w.next[lev];
+          count = w.count[lev];
+          continue;
+        }
+        if (lev > 0) {
+          const uint32_t k = next + slot, child = k < count ? 8u * w.open[lev][k] + oct : 0xFFFFFFFFu;
+          if (lane == 0) {
+            w.next[lev] = (uint8_t)(next + 4u);
+            w.count[lev] = (uint8_t)count;
+          }
+          --lev;
+          bool hit = false;
+          if (child < v.ol.count[lev]) {
+            const float4* b = v.box + 2 * (size_t)(v.ol.first[lev] + child);
+            hit = box_dist2(x, b[0], b[1]) <= q.w;
+          }
+          const uint32_t m = __ballot_sync(0xffffffffu, hit);
+          if (hit) w.open[lev][__popc(m & lt)] = child;
+          next = 0;
+          count = __popc(m);
+          __syncwarp();
+        } else {
+          // up to eight boxes of photons: two rounds' loads together
+          uint32_t leaf[2];
+          float4 p[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const uint32_t k = next + 4u * i + slot;
+            leaf[i] = k < count ? 8u * w.open[0][k] + oct : 0xFFFFFFFFu;
+            if (leaf[i] < n) p[i] = v.leaf_lo[leaf[i]];
+          }
+          next += 8u;
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            bool hit = false;
+            if (leaf[i] < n) {
+              ++cand;
+              const f3 dq = mk(p[i].x, p[i].y, p[i].z) - x;
+              hit = dot(dq, dq) <= q.w;
+            }
+            const uint32_t found = __ballot_sync(0xffffffffu, hit);
+            if (hit) {
+              const uint32_t at = (qh + qn + __popc(found & lt)) & 63u;
+              w.leaf[at] = leaf[i];
+              w.of[at] = (uint8_t)j;
+            }
+            qn += __popc(found);
+            if (lane == j) M += __popc(found);
+            if (qn >= 32u) evaluate();
+          }
+          __syncwarp();
+        }
+      }
+    }
+    if (qn) evaluate();
+    if (lane < here) {
+      phi = sigma_t > 0.0f ? mk(phi.x / sigma_t, phi.y / sigma_t, phi.z / sigma_t) : mk(0.f, 0.f, 0.f);
+      ppm_update(v, s, pix, M, phi, mk(0.f, 0.f, 0.f), sum);
+      found_total += M;
+    }
+    __syncwarp();  // the points are written again
+  }
+  flush_counters(cnt, 0ull, 0ull, found_total, 0ull);
   warp_count(tested, cand);
 }
 
@@ -423,7 +670,7 @@ void ppm_free(vcr_ctx* ctx) {
   void* ptrs[] = {st->pos, st->pw, st->dir, st->uid, st->count, st->by_uid, st->uid_sorted, st->codes, st->idx,
                   st->codes_sorted, st->order, st->left, st->right, st->parent_int, st->parent_leaf, st->flags,
                   st->leaf_lo, st->leaf_hi, st->node_lo, st->node_hi, st->node_pk, st->leaf_pw, st->leaf_dir,
-                  st->stats, st->iota};
+                  st->box, st->stats, st->iota, st->points, st->point, st->point_pix};
   for (void* p : ptrs) cudaFree(p);
   probe_free(st->gather);
   delete st;
@@ -464,17 +711,23 @@ vcr_status ppm_setup(vcr_ctx* ctx, const vcr_ppm_params* p) {
   VCR_ALLOC(st->right, C * 4);
   VCR_ALLOC(st->parent_int, C * 4);
   VCR_ALLOC(st->parent_leaf, C * 4);
-  VCR_ALLOC(st->flags, C * 4);
   VCR_ALLOC(st->leaf_lo, C * 16);
-  VCR_ALLOC(st->leaf_hi, C * 16);
-  VCR_ALLOC(st->node_lo, C * 16);
-  VCR_ALLOC(st->node_hi, C * 16);
-  VCR_ALLOC(st->node_pk, 2 * C * 16);
-  VCR_ALLOC(st->leaf_pw, C * 16);
-  VCR_ALLOC(st->leaf_dir, C * 16);
+  VCR_ALLOC(st->box, (size_t)oct_layout(p->capacity).total * 32 + 8 * 32);  // a visit reads 8 boxes
+  if (p->estimator == VCR_PPM_MARCH) {  // the march walks the tree's boxes and leaf-order photons
+    VCR_ALLOC(st->flags, C * 4);
+    VCR_ALLOC(st->leaf_hi, C * 16);
+    VCR_ALLOC(st->node_lo, C * 16);
+    VCR_ALLOC(st->node_hi, C * 16);
+    VCR_ALLOC(st->node_pk, 2 * C * 16);
+    VCR_ALLOC(st->leaf_pw, C * 16);
+    VCR_ALLOC(st->leaf_dir, C * 16);
+  }
   VCR_ALLOC(st->iota, C * 4);
   size_t px = (size_t)ctx->width * ctx->height;
   VCR_ALLOC(st->stats, px * 8 * sizeof(double));
+  VCR_ALLOC(st->points, 4);
+  VCR_ALLOC(st->point, px * 16);
+  VCR_ALLOC(st->point_pix, px * 4);
 #undef VCR_ALLOC
   iota_kernel<<<(unsigned)((C + 255) / 256), 256>>>(st->iota, (uint32_t)C);
   ppm_init_stats_kernel<<<(unsigned)((px + 255) / 256), 256>>>(st->stats, px, (double)p->radius);
@@ -553,17 +806,45 @@ vcr_status ppm_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
   }
   VCR_CUDA(ctx, sort_pairs_enqueue(ctx->sm_count, ctx->d_error, ctx->d_scratch, st->codes, st->idx,
                                    st->codes_sorted, st->order, n, 0, 30, cs));
-  vs = lbvh_build_refit(ctx, st->codes_sorted, st->order, st->pos, st->pos, (int)n, st->left, st->right,
-                        st->parent_int, st->parent_leaf, st->flags, st->leaf_lo, st->leaf_hi, st->node_lo,
-                        st->node_hi, cs, st->node_pk);
-  if (vs) return vs;
-  if (n) {  // powers and directions in leaf order, read with the leaf's position
-    ppm_leaf_order_kernel<<<ctx->sm_count * 8, 256, 0, cs>>>(st->order, st->pw, st->dir, n, st->leaf_pw,
-                                                             st->leaf_dir);
-    VCR_CUDA(ctx, cudaGetLastError());
+  PpmGatherView gv{};
+  gv.leaf_lo = st->leaf_lo;
+  gv.n = (int)n;
+  gv.stats = st->stats;
+  gv.alpha = st->prm.alpha;
+  gv.seed = pass->seed;
+  gv.pass = pass->pass_index;
+  if (march) {
+    vs = lbvh_build_refit(ctx, st->codes_sorted, st->order, st->pos, st->pos, (int)n, st->left, st->right,
+                          st->parent_int, st->parent_leaf, st->flags, st->leaf_lo, st->leaf_hi, st->node_lo,
+                          st->node_hi, cs, st->node_pk);
+    if (vs) return vs;
+    if (n) {  // powers and directions in leaf order, read with the leaf's position
+      ppm_leaf_order_kernel<<<ctx->sm_count * 8, 256, 0, cs>>>(st->order, st->pw, st->dir, n, st->leaf_pw,
+                                                               st->leaf_dir);
+      VCR_CUDA(ctx, cudaGetLastError());
+    }
+    gv.pw = st->leaf_pw;
+    gv.dir = st->leaf_dir;
+    gv.node_pk = st->node_pk;
+  } else {  // the tree's topology (readable), and the clusters the gather descends
+    vs = lbvh_build(ctx, st->codes_sorted, (int)n, st->left, st->right, st->parent_int, st->parent_leaf, cs);
+    if (vs) return vs;
+    gv.ol = oct_layout(n);
+    uint32_t inputs = n;
+    for (int level = 0; level < gv.ol.levels && n; level += 3) {
+      oct_kernel<<<(inputs + kOctThreads - 1) / kOctThreads, kOctThreads, 0, cs>>>(st->order, st->pos, st->leaf_lo,
+                                                                                 st->box, gv.ol, level, inputs);
+      VCR_CUDA(ctx, cudaGetLastError());
+      for (int k = 0; k < 3; ++k) inputs = (inputs + 7u) / 8u;
+    }
+    gv.pw = st->pw;
+    gv.dir = st->dir;
+    gv.order = st->order;
+    gv.box = st->box;
+    gv.points = st->points;
+    gv.point = st->point;
+    gv.point_pix = st->point_pix;
   }
-  PpmGatherView gv{st->leaf_pw, st->leaf_dir, st->leaf_lo, st->node_pk, (int)n, st->stats, st->prm.alpha, pass->seed,
-                   pass->pass_index};
   uint32_t pixels = pv.cw * pv.ch;
   vcr_status ps = probe_begin(ctx, st->gather, cs);
   if (ps) return ps;
@@ -572,7 +853,13 @@ vcr_status ppm_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
         g, s, cam_view(ctx->cam), sv_view(ctx), pv, gv, ppm_global_radius(st->prm.radius, st->prm.alpha, pv.pass),
         st->prm.march_step, st->prm.ambient_step, ctx->d_sum, cnt, st->gather.d_count);
   } else {
-    ppm_gather_kernel<<<(pixels + 127) / 128, 128, 0, cs>>>(g, s, cam_view(ctx->cam), pv, gv, ctx->d_sum, cnt,
+    VCR_CUDA(ctx, cudaMemsetAsync(st->points, 0, 4, cs));
+    ppm_camera_kernel<<<(pixels + 127) / 128, 128, 0, cs>>>(g, s, cam_view(ctx->cam), pv, gv, ctx->d_sum, cnt);
+    VCR_CUDA(ctx, cudaGetLastError());
+    const uint32_t blocks = std::min<uint32_t>((uint32_t)ctx->sm_count * 8u,
+                                               (pixels + kPpmGatherThreads / 32 * kPpmChunk - 1) /
+                                                   (kPpmGatherThreads / 32 * kPpmChunk));
+    ppm_gather_kernel<<<blocks, kPpmGatherThreads, 0, cs>>>(s, cam_view(ctx->cam), pv, gv, ctx->d_sum, cnt,
                                                             st->gather.d_count);
   }
   VCR_CUDA(ctx, cudaGetLastError());

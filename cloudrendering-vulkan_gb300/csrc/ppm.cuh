@@ -19,9 +19,15 @@ struct PpmState {
            *idx = nullptr, *codes_sorted = nullptr, *order = nullptr, *iota = nullptr;
   uint32_t *left = nullptr, *right = nullptr, *parent_int = nullptr, *parent_leaf = nullptr, *flags = nullptr;
   float4 *leaf_lo = nullptr, *leaf_hi = nullptr, *node_lo = nullptr, *node_hi = nullptr;
-  float4* node_pk = nullptr;   // internal nodes packed for the gather: (lo, left), (hi, right)
-  float4* leaf_pw = nullptr;   // photon powers in leaf order
-  float4* leaf_dir = nullptr;  // photon directions in leaf order
+  // the march's tree walk: internal nodes packed as (lo, left), (hi, right),
+  // photon powers and directions in leaf order
+  float4* node_pk = nullptr;
+  float4* leaf_pw = nullptr;
+  float4* leaf_dir = nullptr;
+  float4* box = nullptr;  // the gather's boxes over 8 consecutive leaves, over 8 of those, ...
+  // the pass's measurement points: their number, position and sigma_t, pixel
+  uint32_t *points = nullptr, *point_pix = nullptr;
+  float4* point = nullptr;
   double* stats = nullptr;  // per pixel: N, R, tau rgb, background rgb
   GatherProbe gather;       // photons the last gather tested, its device time
 };
