@@ -37,6 +37,10 @@ vcr_status lbvh_build_refit(vcr_ctx* ctx, const uint32_t* codes, const uint32_t*
                             uint32_t* parent_leaf, uint32_t* flags, float4* leaf_lo, float4* leaf_hi,
                             float4* node_lo, float4* node_hi, cudaStream_t st, float4* node_pk);
 
+cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* sums, uint32_t* d_total,
+                               cudaStream_t st);
+constexpr uint32_t kPlacePhotons = 1u << 21;  // exclusive_scan_u32's limit
+
 // Photon box entry and power: the same sun / constant-sky emission as the
 // beams (see ppb.cu).
 __device__ __forceinline__ float ppm_box_entry(const SceneView& s, f3 d, Rng& rng, f3& o) {
@@ -57,7 +61,7 @@ __device__ __forceinline__ float ppm_box_entry(const SceneView& s, f3 d, Rng& rn
 // path runs.  Deposits at every real collision go to a shared buffer
 // through one atomic per warp and round (order fixed later by uid; a
 // photon's path, and so every deposit, is the same whichever lane traces
-// it).
+// it).  n_events[p] is the number of photon p's deposits.
 __device__ __forceinline__ void ppm_start_photon(const SceneView& s, uint32_t p, uint32_t photons, uint32_t seed,
                                                  uint32_t pass, Rng& rng, f3& o, f3& d, f3& power) {
   rng = rng_pcg(seed ^ kPpmEmitSalt, p, pass);
@@ -85,7 +89,7 @@ __global__ void __launch_bounds__(128) ppm_emit_kernel(GridView g, SceneView s, 
                                                        uint32_t pass, uint32_t cap, float4* __restrict__ pos,
                                                        float4* __restrict__ pw, float4* __restrict__ dir,
                                                        uint32_t* __restrict__ uid, uint32_t* __restrict__ count,
-                                                       Counters cnt) {
+                                                       uint32_t* __restrict__ n_events, Counters cnt) {
   const uint32_t lane = threadIdx.x & 31u;
   bool alive = false, exhausted = false;
   uint32_t p = 0, events = 0;
@@ -122,6 +126,7 @@ __global__ void __launch_bounds__(128) ppm_emit_kernel(GridView g, SceneView s, 
         dep = true;
       } else {
         alive = false;
+        n_events[p] = events;
       }
     }
     const uint32_t m = __ballot_sync(0xffffffffu, dep);
@@ -141,12 +146,38 @@ __global__ void __launch_bounds__(128) ppm_emit_kernel(GridView g, SceneView s, 
         ++events;
         ++deposits;
         power = power * s.albedo;
-        if ((s.max_events && events >= s.max_events) || events >= kPpmMaxEvents) alive = false;
-        else d = hg_sample(s.ph, d, rng, true);
+        if ((s.max_events && events >= s.max_events) || events >= kPpmMaxEvents) {
+          alive = false;
+          n_events[p] = events;
+        } else {
+          d = hg_sample(s.ph, d, rng, true);
+        }
       }
     }
   }
   flush_counters(cnt, started, lookups, deposits, cells);
+}
+
+__device__ __forceinline__ uint32_t ppm_code(const SceneView& s, float4 p) {
+  f3 e = s.b1 - s.b0;
+  float qx = fminf(fmaxf(((p.x - s.b0.x) / e.x) * 1024.0f, 0.0f), 1023.0f);
+  float qy = fminf(fmaxf(((p.y - s.b0.y) / e.y) * 1024.0f, 0.0f), 1023.0f);
+  float qz = fminf(fmaxf(((p.z - s.b0.z) / e.z) * 1024.0f, 0.0f), 1023.0f);
+  return (morton_expand10((uint32_t)qx) << 2) | (morton_expand10((uint32_t)qy) << 1) | morton_expand10((uint32_t)qz);
+}
+
+// Morton key of each photon in uid order: photon p's event e is number
+// first[p] + e of them (first: the exclusive sums of the photons' deposits).
+// A sort by uid gives the same order in four passes: 150 us for 3.2 M
+// photons, the sums and this kernel 51 us.
+__global__ void ppm_place_kernel(SceneView s, const float4* __restrict__ pos, const uint32_t* __restrict__ uid,
+                                 const uint32_t* __restrict__ first, uint32_t n, uint32_t* __restrict__ codes,
+                                 uint32_t* __restrict__ idx) {
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t u = uid[i], at = first[u / kPpmMaxEvents] + u % kPpmMaxEvents;
+  codes[at] = ppm_code(s, pos[i]);
+  idx[at] = i;
 }
 
 // Morton key of each photon in uid order (order = photons sorted by uid).
@@ -155,13 +186,7 @@ __global__ void ppm_keys_kernel(SceneView s, const float4* __restrict__ pos, con
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t ph = by_uid[i];
-  float4 p = pos[ph];
-  f3 e = s.b1 - s.b0;
-  float qx = fminf(fmaxf(((p.x - s.b0.x) / e.x) * 1024.0f, 0.0f), 1023.0f);
-  float qy = fminf(fmaxf(((p.y - s.b0.y) / e.y) * 1024.0f, 0.0f), 1023.0f);
-  float qz = fminf(fmaxf(((p.z - s.b0.z) / e.z) * 1024.0f, 0.0f), 1023.0f);
-  codes[i] = (morton_expand10((uint32_t)qx) << 2) | (morton_expand10((uint32_t)qy) << 1) |
-             morton_expand10((uint32_t)qz);
+  codes[i] = ppm_code(s, pos[ph]);
   idx[i] = ph;
 }
 
@@ -670,7 +695,8 @@ void ppm_free(vcr_ctx* ctx) {
   void* ptrs[] = {st->pos, st->pw, st->dir, st->uid, st->count, st->by_uid, st->uid_sorted, st->codes, st->idx,
                   st->codes_sorted, st->order, st->left, st->right, st->parent_int, st->parent_leaf, st->flags,
                   st->leaf_lo, st->leaf_hi, st->node_lo, st->node_hi, st->node_pk, st->leaf_pw, st->leaf_dir,
-                  st->box, st->stats, st->iota, st->points, st->point, st->point_pix};
+                  st->box, st->stats, st->iota, st->points, st->point, st->point_pix,
+                  st->deposits, st->first, st->scan_sums};
   for (void* p : ptrs) cudaFree(p);
   probe_free(st->gather);
   delete st;
@@ -723,6 +749,9 @@ vcr_status ppm_setup(vcr_ctx* ctx, const vcr_ppm_params* p) {
     VCR_ALLOC(st->leaf_dir, C * 16);
   }
   VCR_ALLOC(st->iota, C * 4);
+  VCR_ALLOC(st->deposits, (size_t)p->photons * 4);
+  VCR_ALLOC(st->first, (size_t)p->photons * 4);
+  VCR_ALLOC(st->scan_sums, 4096 * 4);
   size_t px = (size_t)ctx->width * ctx->height;
   VCR_ALLOC(st->stats, px * 8 * sizeof(double));
   VCR_ALLOC(st->points, 4);
@@ -785,7 +814,7 @@ vcr_status ppm_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
     VCR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ppm_emit_kernel, 128, 0));
     const uint32_t blocks = std::min<uint32_t>((uint32_t)(ctx->sm_count * std::max(per_sm, 1)), (P + 127) / 128);
     ppm_emit_kernel<<<blocks, 128, 0, cs>>>(g, s, P, pass->seed, pass->pass_index, C, st->pos, st->pw, st->dir,
-                                            st->uid, st->count, cnt);
+                                            st->uid, st->count, st->deposits, cnt);
   }
   VCR_CUDA(ctx, cudaGetLastError());
   uint32_t total = 0;
@@ -795,14 +824,24 @@ vcr_status ppm_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
   st->photons_stored = n;
   st->dropped = total - n;
   // deterministic order: by (photon, event) uid, then stable along the Morton
-  // curve; the uid sort covers only the bits a uid of this photon count uses
-  uint32_t uid_bits = 1;
-  while (uid_bits < 32 && (1ull << uid_bits) <= (uint64_t)P * kPpmMaxEvents + kPpmMaxEvents) ++uid_bits;
-  VCR_CUDA(ctx, sort_pairs_enqueue(ctx->sm_count, ctx->d_error, ctx->d_scratch, st->uid, st->iota, st->uid_sorted,
-                                   st->by_uid, n, 0, uid_bits, cs));
-  if (n) {
-    ppm_keys_kernel<<<(n + 255) / 256, 256, 0, cs>>>(s, st->pos, st->by_uid, n, st->codes, st->idx);
-    VCR_CUDA(ctx, cudaGetLastError());
+  // curve
+  if (total <= C && P <= kPlacePhotons) {
+    VCR_CUDA(ctx, exclusive_scan_u32(st->deposits, st->first, P, st->scan_sums, nullptr, cs));
+    if (n) {
+      ppm_place_kernel<<<(n + 255) / 256, 256, 0, cs>>>(s, st->pos, st->uid, st->first, n, st->codes, st->idx);
+      VCR_CUDA(ctx, cudaGetLastError());
+    }
+  } else {
+    // more photons than the scan takes, or deposits that were dropped: a sort
+    // by uid, over the bits a uid of this photon count uses
+    uint32_t uid_bits = 1;
+    while (uid_bits < 32 && (1ull << uid_bits) <= (uint64_t)P * kPpmMaxEvents + kPpmMaxEvents) ++uid_bits;
+    VCR_CUDA(ctx, sort_pairs_enqueue(ctx->sm_count, ctx->d_error, ctx->d_scratch, st->uid, st->iota, st->uid_sorted,
+                                     st->by_uid, n, 0, uid_bits, cs));
+    if (n) {
+      ppm_keys_kernel<<<(n + 255) / 256, 256, 0, cs>>>(s, st->pos, st->by_uid, n, st->codes, st->idx);
+      VCR_CUDA(ctx, cudaGetLastError());
+    }
   }
   VCR_CUDA(ctx, sort_pairs_enqueue(ctx->sm_count, ctx->d_error, ctx->d_scratch, st->codes, st->idx,
                                    st->codes_sorted, st->order, n, 0, 30, cs));
