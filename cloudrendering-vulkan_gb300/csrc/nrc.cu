@@ -29,10 +29,11 @@ namespace vcr {
 
 using bf16 = __nv_bfloat16;
 
-// Training CTA: 8 warps, 16 records each, one 128-record tile at a time.
-constexpr int kTrainWarps = 8;
-constexpr int kTrainThreads = kTrainWarps * 32;
-constexpr int kTrainTile = kTrainWarps * 16;
+// Training CTA: 4 chain warps (forward and backward, 32 records each), 4
+// gradient warps and 4 encoder warps, one 128-record tile at a time.
+constexpr int kTrainRole = 4 * 32;  // threads of a role
+constexpr int kTrainThreads = 3 * kTrainRole;
+constexpr int kTrainTile = 128;
 
 constexpr int kTileX = kTrainTile * kLdX;                                  // one activation tile
 
@@ -106,34 +107,192 @@ __global__ void __launch_bounds__(kInferThreads, 3) nrc_infer_kernel(NrcView v, 
 // training: relative L2 loss sum_c (y - t)^2 / (sg(y)^2 + 0.01) / (3 B)
 // ---------------------------------------------------------------------------
 
-// The lane's four BF16 pairs of an A fragment (rows g, g+8; columns 2t and
-// 8+2t of each 16-column tile kt) to / from a [record][feature] tile with
-// kLdX rows: 4-byte accesses on 32 distinct banks.
-__device__ __forceinline__ void store_a(bf16* T, int row, int t, const uint32_t (&a)[4][4], int tiles) {
+// Launched with launch_overlapped, a kernel may be set up on the device while
+// the one before it in its stream still runs; grid_wait waits for that one's
+// end, and comes before any access to memory.  grid_trigger lets the next one
+// be set up.  A training step is two short kernels: 41.7 -> 41.0 us.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+
+// Registers a thread of each role, a launch with 168 in all: 3 x 168 = 504.
+constexpr int kRegsChain = 216, kRegsGrad = 224, kRegsEncode = 64;
+static_assert(kRegsChain + kRegsGrad + kRegsEncode <= 3 * 168, "register split");
+template <int kRegs>
+__device__ __forceinline__ void set_regs_up() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs));
+}
+template <int kRegs>
+__device__ __forceinline__ void set_regs_down() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
+}
+
+// k-tile kt of the B fragments of a hidden layer, W_l as [in][out] (the
+// forward) and as [out][in] (the backward); NP 16-wide tiles.
+template <int NP>
+__device__ __forceinline__ void load_in_out(const bf16* Wl, int ld, int kt, uint32_t (&b)[4][4], int lane) {
+  const int rr = lane & 7, q = lane >> 3;
+#pragma unroll
+  for (int np = 0; np < NP; ++np) ldsm_x4_t(b[np], Wl + (kt * 16 + rr + 8 * (q & 1)) * ld + np * 16 + 8 * (q >> 1));
+}
+__device__ __forceinline__ void load_out_in(const bf16* Wl, int ld, int kt, uint32_t (&b)[4][4], int lane) {
+  const int rr = lane & 7, q = lane >> 3;
+#pragma unroll
+  for (int np = 0; np < 4; ++np) ldsm_x4(b[np], Wl + (np * 16 + rr + 8 * (q >> 1)) * ld + kt * 16 + 8 * (q & 1));
+}
+
+// mma_bf16 with zero for the accumulators' old values.
+__device__ __forceinline__ void mma_bf16_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%10,%10,%10,%10};\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+}
+
+// One layer of one fragment of 16 records, acc = a b over KT k-tiles.  After
+// each pair of MMAs comes other(kt, np), a sixteenth of what the last layer of
+// the warp's other fragment leaves to do: its scalar work fills the issue
+// slots between the MMAs.  After k-tile kt comes reload(kt), for b[kt] is not
+// needed any more.
+template <int KT, class Reload, class Other>
+__device__ __forceinline__ void chain_phase(float (&acc)[8][4], const uint32_t (&a)[4][4], uint32_t (&b)[4][4][4],
+                                            Reload reload, Other other) {
 #pragma unroll
   for (int kt = 0; kt < 4; ++kt) {
-    if (kt >= tiles) break;
-    uint32_t* p0 = reinterpret_cast<uint32_t*>(T + row * kLdX + kt * 16 + 2 * t);
-    uint32_t* p1 = reinterpret_cast<uint32_t*>(T + (row + 8) * kLdX + kt * 16 + 2 * t);
-    p0[0] = a[kt][0];
-    p1[0] = a[kt][1];
-    p0[4] = a[kt][2];
-    p1[4] = a[kt][3];
+#pragma unroll
+    for (int np = 0; np < 4; ++np) {
+      if (kt == 0) {
+        mma_bf16_zero(acc[2 * np], a[kt], b[kt][np][0], b[kt][np][1]);
+        mma_bf16_zero(acc[2 * np + 1], a[kt], b[kt][np][2], b[kt][np][3]);
+      } else if (kt < KT) {
+        mma_bf16(acc[2 * np], a[kt], b[kt][np][0], b[kt][np][1]);
+        mma_bf16(acc[2 * np + 1], a[kt], b[kt][np][2], b[kt][np][3]);
+      }
+      other(kt, np);
+    }
+    reload(kt);
   }
 }
 
-// One 8-warp CTA per SM; a 128-record tile at a time, 16 records per warp.
-// The forward keeps a warp's activations in its MMA fragments (as the
-// queries do) and stores each layer's input X_l once, as BF16, into the
-// tile's shared [record][feature] buffers; the backward runs dY_l W_l^T in
-// registers as well (the dY A fragments of one layer are the masked
-// accumulators of the last), so only X_l and dY_l go through shared memory,
-// for the weight gradient dW_l = X_l^T dY_l over all 128 records.  Warp w
-// owns the 16 x 32 block (rows 16(w/2).., columns 32(w%2)..) of every 64x64
-// hidden-layer gradient and the 16 x 8 block (rows 16(w/2).., columns
-// 8(w%2)..) of the 64x16 output layer's, in registers across the CTA's
-// tiles; X_l^T and dY_l fragments come from ldmatrix.trans.  At the end each
-// CTA stores its gradient into its own slot of gpart.
+// Word p of k-tile kt of a fragment to its rows of a tile.
+__device__ __forceinline__ void store_word(bf16* T, int row, int t, int kt, int p, uint32_t w) {
+  *reinterpret_cast<uint32_t*>(T + (row + 8 * (p & 1)) * kLdX + kt * 16 + 8 * (p >> 1) + 2 * t) = w;
+}
+
+// ReLU and BF16 of word p of accumulator tiles 2 kt, 2 kt + 1: the A fragment
+// of the next layer's k-tile kt (the maximum after the rounding is the
+// rounding of the maximum, and takes a NaN to 0 like fmaxf).
+__device__ __forceinline__ uint32_t relu_word(const float (&acc)[8][4], int kt, int p) {
+  const float* y = &acc[2 * kt + (p >> 1)][2 * (p & 1)];
+  const __nv_bfloat162 r = __hmax2(__floats2bfloat162_rn(y[0], y[1]), __floats2bfloat162_rn(0.0f, 0.0f));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+// The same for the backward: the accumulators times 1 where the layer's input
+// x is above zero, else times 0.
+__device__ __forceinline__ uint32_t mask_word(const float (&acc)[8][4], int kt, int p, uint32_t x) {
+  const float* y = &acc[2 * kt + (p >> 1)][2 * (p & 1)];
+  const __nv_bfloat162 one = __hgt2(*reinterpret_cast<const __nv_bfloat162*>(&x), __floats2bfloat162_rn(0.0f, 0.0f));
+  const __nv_bfloat162 r = __hmul2(__floats2bfloat162_rn(y[0], y[1]), one);
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+// A fragment of 16 records of a [record][feature] tile, by the address of the
+// lane's row of it.
+__device__ __forceinline__ void load_fragment(const bf16* p, uint32_t (&a)[4][4]) {
+#pragma unroll
+  for (int kt = 0; kt < 4; ++kt) ldsm_x4(a[kt], p + kt * 16);
+}
+
+// Half of the 64 inputs of one record as its row of X_0 (nrc_encode's order):
+// eight levels and one direction; zeros for a row without a record.
+template <bool kGrid>
+__device__ __forceinline__ void encode_half(const NrcRecord* rec, int half, const NrcView& v, const float* dirs,
+                                            bf16* row) {
+  uint4* out = reinterpret_cast<uint4*>(row) + 2 * half;
+  if (!rec) {
+    out[0] = out[1] = out[4] = out[5] = make_uint4(0u, 0u, 0u, 0u);
+    return;
+  }
+  float ux, uy, uz;
+  nrc_box_coords(*rec, v.b0, v.inv_ext, ux, uy, uz);
+  const float* d = half ? &rec->sx : &rec->vx;
+  const float dx = d[0], dy = d[1], dz = d[2];
+#pragma unroll 1
+  for (int j = 0; j < 2; ++j) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int l = 8 * half + 4 * j + i;
+      float sn = 0.0f, cs = 0.0f;
+      if (l < v.levels) {
+        if (kGrid) nrc_grid_level(v.gtab, l, ux, uy, uz, &sn, &cs);
+        else nrc_encode_level_dir(l, dirs[3 * l], dirs[3 * l + 1], dirs[3 * l + 2], ux, uy, uz, &sn, &cs);
+      }
+      w[i] = pack_bf16(sn, cs);
+    }
+    out[j] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  float sh[16];
+  nrc_sh16(dx, dy, dz, sh);
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    out[4 + j] = make_uint4(pack_bf16(sh[8 * j], sh[8 * j + 1]), pack_bf16(sh[8 * j + 2], sh[8 * j + 3]),
+                            pack_bf16(sh[8 * j + 4], sh[8 * j + 5]), pack_bf16(sh[8 * j + 6], sh[8 * j + 7]));
+}
+
+// Named barriers of the training CTA (0 is __syncthreads).  Each is arrived
+// at by one role and waited for by another; a pair is used in turn, so a role
+// never arrives twice at one barrier before the other has passed it.
+enum TrainBar : int {
+  kBarFull = 1,   // +0, +1: dY_l (and X_l) of every row stored; chain -> gradient
+  kBarEmpty = 3,  // +0, +1: dW_l added up, its dY buffer and X_l free; gradient -> chain
+  kBarInput = 5,  // +0, +1: X_0 of a tile encoded; encoders -> chain
+  kBarSpare = 7,  // +0, +1: dW_0 added up, its buffer of X_0 free; gradient -> encoders
+  kBarFirst = 9,  // X_0 of the first tile; encoders and gradient -> chain
+  kBarDirs = 10,  // the level directions; encoders and gradient
+  kBarChain = 11, // the weights; the chain warps alone
+};
+template <int kRoles>
+__device__ __forceinline__ void bar_arrive(int id) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kRoles * kTrainRole) : "memory");
+}
+template <int kRoles>
+__device__ __forceinline__ void bar_wait(int id) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kRoles * kTrainRole) : "memory");
+}
+
+// One CTA per SM, a 128-record tile at a time, in three roles of 4 warps, one
+// of each on every scheduler.
+//
+// Chain warps own 32 records each, as two fragments of 16 that are half a
+// layer apart: while the tensor pipe works on one, the other's activations
+// are rounded and stored.  The forward keeps the activations in MMA fragments
+// (as the queries do) and stores each layer's input X_l once, as BF16, into
+// the tile's shared [record][feature] buffers; the backward runs dY_l W_l^T
+// in registers as well (the dY A fragments of one layer are the masked
+// accumulators of the last), so only X_l and dY_l go
+// through shared memory.
+//
+// Gradient warps add up dW_l = X_l^T dY_l over all 128 records as soon as
+// dY_l is stored, while the chain warps work on dY_{l-1}.  Warp w owns the
+// 32 x 32 block (rows 32(w/2).., columns 32(w%2)..) of every 64x64
+// hidden-layer gradient and rows 16w.. of the 64x16 output layer's, in
+// registers across the CTA's tiles; X_l^T and dY_l fragments come from
+// ldmatrix.trans.  At the end each CTA stores its gradient into its own slot
+// of gpart.
+//
+// Encoder warps write the next tile's inputs, a record a lane (X_0 has two
+// buffers).
+//
+// What bounds it: a tile's 3,840 MMAs take 7,700 cycles of the four tensor
+// pipes (8.1 each; FMA-pipe instructions go to the same port, so the masks and
+// maxima are packed BF16), its operands 9,600 wavefronts of shared memory; it
+// takes 13,300 cycles, the forward at the chain's latency, the backward at
+// both pipes (1,500 cycles a layer).  65,536 records, 8 steps: 431 us with
+// eight warps that did everything in turn (two barriers a layer, 11,200
+// wavefronts a tile), 382 with eight chain and eight gradient warps, 333 so
+// (348 with eight gradient warps of half the block: more wavefronts).
 //
 // kGrid (the grid encoding): the backward also forms dX_0 = dY_0 W_0^T for
 // the 32 position inputs in registers and adds, for every record, level and
@@ -146,157 +305,306 @@ __global__ void __launch_bounds__(kTrainThreads, 1) nrc_train_kernel(NrcView v, 
                                                                      float* __restrict__ gpart, float* __restrict__ loss) {
   extern __shared__ __align__(128) unsigned char smem[];
   bf16* W = reinterpret_cast<bf16*>(smem);              // [in][out], rows of ldw(l)
-  bf16* X = W + kWs;                                     // X_0 .. X_5 of the tile
-  bf16* D = X + kNrcLayers * kTileX;                     // dY ping-pong: 2 tiles
+  bf16* X = W + kWs;                                     // X_1 .. X_5 of the tile at l * kTileX, X_0 of two tiles at 0 and 6
+  bf16* D = X + (kNrcLayers + 1) * kTileX;               // dY ping-pong: dY_5, dY_3, dY_1 in buffer 0
   float* dirs = reinterpret_cast<float*>(D + 2 * kTileX);  // 16 position-level directions
   // records [first_rec, first_rec + capacity) of the *count_ptr written; a
   // CTA without a tile leaves its slot alone (the reduction reads the slots
   // of the first ceil(count / kTrainTile) CTAs only)
+  grid_wait();
+  grid_trigger();
   const uint32_t total = *count_ptr;
+  const int role = threadIdx.x / kTrainRole;  // 0 chain, 1 gradient, 2 encoders
+  const int k = threadIdx.x & (kTrainRole - 1);
+  // what does not depend on the records, while the count is on its way
+  if (role == 0) {
+    load_weights<kTrainRole>(v.wb, W);
+    bar_wait<1>(kBarChain);
+  } else {
+    if (role == 2 && k < kNrcPosLevels) nrc_level_dir(k, dirs[3 * k], dirs[3 * k + 1], dirs[3 * k + 2]);
+    bar_wait<2>(kBarDirs);
+  }
   const uint32_t count = total > first_rec ? min(total - first_rec, capacity) : 0u;
   if (blockIdx.x * kTrainTile >= count) return;
-  load_weights<kTrainThreads>(v.wb, W);
-  load_level_dirs(dirs);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int rr = lane & 7, q = lane >> 3;
-  const int mt = warp >> 1, half = warp & 1;  // the warp's gradient blocks
-  float dwh[kNrcHidden][4][4], dwo[4];
-#pragma unroll
-  for (int l = 0; l < kNrcHidden; ++l)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) dwh[l][j][0] = dwh[l][j][1] = dwh[l][j][2] = dwh[l][j][3] = 0.0f;
-  dwo[0] = dwo[1] = dwo[2] = dwo[3] = 0.0f;
-  __syncthreads();
+  const uint32_t start = blockIdx.x * kTrainTile, stride = gridDim.x * kTrainTile;
   recs += first_rec;
+
+  if (role == 2) {
+    set_regs_down<kRegsEncode>();
+    uint32_t tile = 0;
+#pragma unroll 1
+    for (uint32_t first = start; first < count; first += stride, ++tile) {
+      const int at = tile & 1;
+      if (tile >= 2) bar_wait<2>(kBarSpare + at);  // dW_0 of the tile before the last
+      const uint32_t idx = first + (uint32_t)k;
+      const NrcRecord* rec = idx < count ? recs + idx : nullptr;
+      bf16* out = X + (at ? kNrcLayers * kTileX : 0) + k * kLdX;
+#pragma unroll 1
+      for (int half = 0; half < (tile ? 2 : 1); ++half) encode_half<kGrid>(rec, half, v, dirs, out);
+      if (tile) bar_arrive<2>(kBarInput + at);
+      else bar_arrive<3>(kBarFirst);
+    }
+    return;
+  }
+
+  if (role == 1) {
+    set_regs_up<kRegsGrad>();
+    // half of the first tile's inputs: there is nothing else to do yet
+    encode_half<kGrid>(start + (uint32_t)k < count ? recs + start + k : nullptr, 1, v, dirs, X + k * kLdX);
+    bar_arrive<3>(kBarFirst);
+    const int m0 = (warp >> 1) * 32, n0 = (warp & 1) * 32;  // the warp's gradient blocks
+    float dwh[kNrcHidden][2][4][4], dwo[2][4];
+#pragma unroll
+    for (int l = 0; l < kNrcHidden; ++l)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          dwh[l][i][j][0] = dwh[l][i][j][1] = dwh[l][i][j][2] = dwh[l][i][j][3] = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) dwo[j][0] = dwo[j][1] = dwo[j][2] = dwo[j][3] = 0.0f;
+    uint32_t tile = 0;
+#pragma unroll 1
+    for (uint32_t first = start; first < count; first += stride, ++tile) {
+      const int at = tile & 1;
+      const bool more = count - first > stride;                     // a next tile
+      const bool spare = more && count - first - stride > stride;  // and one after it
+#pragma unroll
+      for (int l = kNrcLayers - 1; l >= 0; --l) {  // unrolled: the gradient blocks are indexed by layer
+        const int buf = (kNrcLayers - 1 - l) & 1;
+        const bf16* Xl = X + (l == 0 && at ? kNrcLayers : l) * kTileX;
+        const bf16* Dl = D + buf * kTileX;
+        bar_wait<2>(kBarFull + buf);  // X_l and dY_l complete for every row
+        // dW_l += X_l^T dY_l over the tile's 128 records (k); the fragments of
+        // 16 records are loaded while the last 16's are used
+        // X_l^T: features by records 16kt..; dY_l: records 16kt.. by columns
+        const bf16* xr = Xl + (rr + 8 * (q >> 1)) * kLdX + 8 * (q & 1) + (l == kNrcLayers - 1 ? warp * 16 : m0);
+        const bf16* dr = Dl + (rr + 8 * (q & 1)) * kLdX + 8 * (q >> 1) + (l == kNrcLayers - 1 ? 0 : n0);
+        uint32_t xa[2][2][4], b[2][2][4];
+        auto load = [&](int kt) {
+#pragma unroll
+          for (int i = 0; i < (l == kNrcLayers - 1 ? 1 : 2); ++i) {
+            ldsm_x4_t(xa[kt & 1][i], xr + kt * 16 * kLdX + 16 * i);
+            ldsm_x4_t(b[kt & 1][i], dr + kt * 16 * kLdX + 16 * i);
+          }
+        };
+        load(0);
+#pragma unroll
+        for (int kt = 0; kt < kTrainTile / 16; ++kt) {
+          if (kt + 1 < kTrainTile / 16) load(kt + 1);
+          const int u = kt & 1;
+          if (l == kNrcLayers - 1) {
+            mma_bf16(dwo[0], xa[u][0], b[u][0][0], b[u][0][1]);
+            mma_bf16(dwo[1], xa[u][0], b[u][0][2], b[u][0][3]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                mma_bf16(dwh[l < kNrcHidden ? l : 0][i][j], xa[u][i], b[u][j >> 1][2 * (j & 1)],
+                         b[u][j >> 1][2 * (j & 1) + 1]);
+          }
+        }
+        if (l > 1 || more) bar_arrive<2>(kBarEmpty + buf);  // nobody waits for the CTA's last two
+      }
+      if (spare) bar_arrive<2>(kBarSpare + at);
+    }
+    // the CTA's gradient ([in][out] layout per layer) into its own slot of
+    // gpart, every weight written (the warps' blocks cover each layer once);
+    // nrc_grad_reduce_kernel sums the slots in a fixed order
+    float* slot = gpart + (size_t)blockIdx.x * kNrcWeightCount;
+#pragma unroll
+    for (int l = 0; l < kNrcHidden; ++l)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float* base = slot + nrc_layer_offset(l) + (m0 + 16 * i + g) * kNrcWidth + n0 + j * 8 + 2 * t;
+          *reinterpret_cast<float2*>(base) = make_float2(dwh[l][i][j][0], dwh[l][i][j][1]);
+          *reinterpret_cast<float2*>(base + 8 * kNrcWidth) = make_float2(dwh[l][i][j][2], dwh[l][i][j][3]);
+        }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      float* base = slot + nrc_layer_offset(kNrcHidden) + (warp * 16 + g) * kNrcOutPad + j * 8 + 2 * t;
+      *reinterpret_cast<float2*>(base) = make_float2(dwo[j][0], dwo[j][1]);
+      *reinterpret_cast<float2*>(base + 8 * kNrcOutPad) = make_float2(dwo[j][2], dwo[j][3]);
+    }
+    return;
+  }
+
+  // chain warps
+  set_regs_up<kRegsChain>();
+  const bf16* xf = X + (warp * 32 + rr + 8 * (q & 1)) * kLdX + 8 * (q >> 1);  // the lane's rows of its warp's fragments
+  const int row = warp * 32 + g;  // the lane's tile rows: row + 8 h, h = 0 .. 3 (fragment h / 2)
   const float inv_n = 1.0f / (3.0f * (float)max(count, 1u));
   float loss_local = 0.0f;
-  const int row = warp * 16 + g;  // the lane's tile rows: row and row + 8
-  for (uint32_t first = blockIdx.x * kTrainTile; first < count; first += gridDim.x * kTrainTile) {
-    const uint32_t i0 = first + (uint32_t)row, i1 = i0 + 8u;
-    uint32_t a[4][4];
-    {
-      NrcRecord r0{}, r1{};
-      if (i0 < count) r0 = recs[i0];
-      if (i1 < count) r1 = recs[i1];
-      encode_a(r0, i0 < count, v.b0, v.inv_ext, dirs, t, 0, a, v.levels, kGrid ? v.gtab : nullptr);
-      encode_a(r1, i1 < count, v.b0, v.inv_ext, dirs, t, 1, a, v.levels, kGrid ? v.gtab : nullptr);
-    }
-    store_a(X, row, t, a, 4);
+  uint32_t tile = 0;
 #pragma unroll 1
-    for (int l = 0; l < kNrcHidden; ++l) {
-      float acc[8][4];
-      mma_layer_in_out<8>(W + woff(l), ldw(l), a, acc, lane);
-      relu_to_a(acc, a);
-      store_a(X + (l + 1) * kTileX, row, t, a, 4);
+  for (uint32_t first = start; first < count; first += stride, ++tile) {
+    const int at = tile & 1;
+    // the targets of the lane's output columns, for the loss below
+    float target[4][2];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const float* tp = &recs[min(first + (uint32_t)row + 8u * h, count - 1u)].w0;
+      target[h][0] = tp[t == 1 ? 2 : 0];
+      target[h][1] = tp[1];
     }
-    // output layer and the loss gradient dY_5 (columns 0..2 of 16)
-    uint32_t da[4][4];
+    if (tile) bar_wait<2>(kBarInput + at);
+    else bar_wait<3>(kBarFirst);
+    uint32_t a[2][4][4];
+    load_fragment(xf + (at ? kNrcLayers : 0) * kTileX, a[0]);
+    load_fragment(xf + (at ? kNrcLayers : 0) * kTileX + 16 * kLdX, a[1]);
+    uint32_t b[4][4][4];
+    float acc[2][8][4];
+    const auto none = [](int, int = 0) {};
+#pragma unroll
+    for (int kt = 0; kt < 4; ++kt) load_in_out<4>(W, ldw(0), kt, b[kt], lane);
+    chain_phase<4>(acc[0], a[0], b, none, none);
+    if (tile > 0) bar_wait<2>(kBarEmpty + 0);  // the last tile's dW_1: X_1 .. X_5 and dY buffer 0 are free
+    // turn l: fragment 1's layer l, then fragment 0's layer l + 1
+#pragma unroll 1
+    for (int l = 0; l < kNrcHidden - 1; ++l) {
+      bf16* Xn = X + (l + 1) * kTileX;
+      chain_phase<4>(
+          acc[1], a[1], b, [&](int kt) { load_in_out<4>(W + woff(l + 1), ldw(0), kt, b[kt], lane); },
+          [&](int kt, int p) {
+            a[0][kt][p] = relu_word(acc[0], kt, p);
+            store_word(Xn, row, t, kt, p, a[0][kt][p]);
+          });
+      chain_phase<4>(acc[0], a[0], b, none, [&](int kt, int p) {
+        a[1][kt][p] = relu_word(acc[1], kt, p);
+        store_word(Xn, row + 16, t, kt, p, a[1][kt][p]);
+      });
+    }
     {
-      float out[2][4];
-      mma_layer_in_out<2>(W + woff(kNrcHidden), ldw(kNrcHidden), a, out, lane);
+      bf16* Xn = X + kNrcHidden * kTileX;
+      chain_phase<4>(
+          acc[1], a[1], b, [&](int kt) { load_in_out<1>(W + woff(kNrcHidden), ldw(kNrcHidden), kt, b[kt], lane); },
+          [&](int kt, int p) {
+            a[0][kt][p] = relu_word(acc[0], kt, p);
+            store_word(Xn, row, t, kt, p, a[0][kt][p]);
+          });
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        a[1][i >> 2][i & 3] = relu_word(acc[1], i >> 2, i & 3);
+        store_word(Xn, row + 16, t, i >> 2, i & 3, a[1][i >> 2][i & 3]);
+      }
+    }
+    // output layer (columns 0..7 of 16: the rest is padding) and the loss
+    // gradient dY_5 (columns 0..2)
+    float out[2][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      out[m][0] = out[m][1] = out[m][2] = out[m][3] = 0.0f;
+#pragma unroll
+      for (int kt = 0; kt < 4; ++kt) mma_bf16(out[m], a[m][kt], b[kt][0][0], b[kt][0][1]);
+    }
+    load_out_in(W + woff(kNrcHidden), ldw(kNrcHidden), 0, b[0], lane);
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
       float d5[4];  // (row, 2t), (row, 2t+1), (row+8, 2t), (row+8, 2t+1)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const uint32_t idx = h ? i1 : i0;
+        const uint32_t idx = first + (uint32_t)row + 16u * m + 8u * h;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int c = 2 * t + e;
           float gval = 0.0f;
           if (c < kNrcOut && idx < count) {
-            const NrcRecord& rec = recs[idx];
-            const float tv = c == 0 ? rec.w0 : (c == 1 ? rec.w1 : rec.w2);
-            const float y = out[0][2 * h + e];
+            const float y = out[m][2 * h + e];
             const float den = y * y + 0.01f;
-            const float diff = y - tv;
-            loss_local += (diff * diff / den) * inv_n;
-            gval = (2.0f * diff / den) * inv_n;
+            const float diff = y - target[2 * m + h][e];
+            const float rel = diff / den;
+            loss_local += (diff * rel) * inv_n;
+            gval = (2.0f * rel) * inv_n;
           }
           d5[2 * h + e] = gval;
         }
       }
-      da[0][0] = pack_bf16(d5[0], d5[1]);
-      da[0][1] = pack_bf16(d5[2], d5[3]);
-      da[0][2] = 0u;  // columns 8..15: padding
-      da[0][3] = 0u;
-      store_a(D, row, t, da, 1);  // dY_5 in buffer 0
+      a[m][0][0] = pack_bf16(d5[0], d5[1]);
+      a[m][0][1] = pack_bf16(d5[2], d5[3]);
+      a[m][0][2] = 0u;  // columns 8..15: padding
+      a[m][0][3] = 0u;
+#pragma unroll
+      for (int p = 0; p < 4; ++p) store_word(D, row + 16 * m, t, 0, p, a[m][0][p]);  // dY_5 in buffer 0
     }
-    // backward through layers 5..0 (unrolled: the gradient blocks are indexed by layer)
+    bar_arrive<2>(kBarFull + 0);
+    // backward, from here a holds dY: dY_{l-1} = (dY_l W_l^T) * (X_l > 0) for
+    // the warp's rows; layer 5 has one k-tile
+    chain_phase<1>(acc[0], a[0], b, none, none);
+    if (tile > 0) bar_wait<2>(kBarEmpty + 1);  // the last tile's dW_0
+    {
+      uint32_t x[4][4];  // X_5
+      load_fragment(xf + kNrcHidden * kTileX, x);
+      chain_phase<1>(
+          acc[1], a[1], b, [&](int kt) { load_out_in(W + woff(kNrcHidden - 1), ldw(0), kt, b[kt], lane); },
+          [&](int kt, int p) {
+            a[0][kt][p] = mask_word(acc[0], kt, p, x[kt][p]);
+            store_word(D + kTileX, row, t, kt, p, a[0][kt][p]);
+          });
+    }
+    // turn l: dY_{l-1} of fragment 0, while dY_l of fragment 1 is finished,
+    // then dY_{l-1} of fragment 1
+#pragma unroll 1
+    for (int l = kNrcHidden - 1; l >= 1; --l) {
+      const int buf = (kNrcLayers - l) & 1;  // of dY_{l-1}
+      uint32_t x[4][4];  // X_{l+1} of fragment 1, then X_l of fragment 0
+      load_fragment(xf + (l + 1) * kTileX + 16 * kLdX, x);
+      chain_phase<4>(acc[0], a[0], b, none, [&](int kt, int p) {
+        a[1][kt][p] = mask_word(acc[1], kt, p, x[kt][p]);
+        store_word(D + (buf ^ 1) * kTileX, row + 16, t, kt, p, a[1][kt][p]);
+      });
+      load_fragment(xf + l * kTileX, x);
+      bar_arrive<2>(kBarFull + (buf ^ 1));  // dY_l
+      bar_wait<2>(kBarEmpty + buf);         // the buffer's last reader, dW_{l+1}
+      chain_phase<4>(
+          acc[1], a[1], b,
+          [&](int kt) {
+            if (l > 1) load_out_in(W + woff(l - 1), ldw(0), kt, b[kt], lane);
+          },
+          [&](int kt, int p) {
+            a[0][kt][p] = mask_word(acc[0], kt, p, x[kt][p]);
+            store_word(D + buf * kTileX, row, t, kt, p, a[0][kt][p]);
+          });
+    }
+    {
+      uint32_t x[4][4];  // X_1
+      load_fragment(xf + kTileX + 16 * kLdX, x);
 #pragma unroll
-    for (int l = kNrcLayers - 1; l >= 0; --l) {
-      const bf16* Xl = X + l * kTileX;
-      const bf16* Dl = D + ((kNrcLayers - 1 - l) & 1) * kTileX;  // dY_5 in buffer 0, dY_4 in 1, ...
-      __syncthreads();                                           // X_l and dY_l complete for every row
-      // dW_l += X_l^T dY_l over the tile's 128 records (k)
-#pragma unroll 2
-      for (int kt = 0; kt < kTrainTile / 16; ++kt) {
-        uint32_t xa[4];  // X_l^T rows 16mt.. (features), columns 16kt.. (records)
-        ldsm_x4_t(xa, Xl + (kt * 16 + rr + 8 * (q >> 1)) * kLdX + mt * 16 + 8 * (q & 1));
-        if (l == kNrcLayers - 1) {
-          uint32_t b[2];  // dY_5 records 16kt.., columns 8 half..
-          ldsm_x2_t(b, Dl + (kt * 16 + rr + 8 * (q & 1)) * kLdX + half * 8);
-          mma_bf16(dwo, xa, b[0], b[1]);
-        } else {
-#pragma unroll
-          for (int np = 0; np < 2; ++np) {
-            uint32_t b[4];  // dY_l records 16kt.., columns 32 half + 16 np ..
-            ldsm_x4_t(b, Dl + (kt * 16 + rr + 8 * (q & 1)) * kLdX + half * 32 + np * 16 + 8 * (q >> 1));
-            mma_bf16(dwh[l < kNrcHidden ? l : 0][2 * np], xa, b[0], b[1]);
-            mma_bf16(dwh[l < kNrcHidden ? l : 0][2 * np + 1], xa, b[2], b[3]);
-          }
-        }
+      for (int i = 0; i < 16; ++i) {
+        a[1][i >> 2][i & 3] = mask_word(acc[1], i >> 2, i & 3, x[i >> 2][i & 3]);
+        store_word(D + kTileX, row + 16, t, i >> 2, i & 3, a[1][i >> 2][i & 3]);  // dY_0 in buffer 1
       }
-      if (l > 0) {
-        // dY_{l-1} = (dY_l W_l^T) * (X_l > 0) for the warp's rows, in registers
-        const bf16* Wl = W + woff(l);
-        const int ld = ldw(l), ktiles = nrc_layer_cols(l) / 16;
-        float acc[8][4];
+      bar_arrive<2>(kBarFull + 1);
+    }
+    if (kGrid) {
+      // dX_0 for inputs 0..31 (n-tiles 0..3): acc[nt] holds (row, 8nt+2t+e)
+      // and (row+8, 8nt+2t+e), i.e. level 4nt+t, feature e
+      const bf16* W0 = W + woff(0);
+#pragma unroll 1
+      for (int m = 0; m < 2; ++m) {
+        float dx[4][4];
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
-#pragma unroll
-        for (int kt = 0; kt < 4; ++kt) {
-          if (kt >= ktiles) break;
-#pragma unroll
-          for (int np = 0; np < 4; ++np) {
-            uint32_t b[4];  // W_l rows (in) 16np.., columns (out) 16kt..: (in, out), (in, out+8), (in+8, out), (in+8, out+8)
-            ldsm_x4(b, Wl + (np * 16 + rr + 8 * (q >> 1)) * ld + kt * 16 + 8 * (q & 1));
-            mma_bf16(acc[2 * np], da[kt], b[0], b[1]);
-            mma_bf16(acc[2 * np + 1], da[kt], b[2], b[3]);
-          }
-        }
-        bf16* Dn = D + ((kNrcLayers - l) & 1) * kTileX;
+        for (int nt = 0; nt < 4; ++nt) dx[nt][0] = dx[nt][1] = dx[nt][2] = dx[nt][3] = 0.0f;
 #pragma unroll
         for (int kt = 0; kt < 4; ++kt) {
-          const uint32_t* h0 = reinterpret_cast<const uint32_t*>(Xl + row * kLdX + kt * 16 + 2 * t);
-          const uint32_t* h1 = reinterpret_cast<const uint32_t*>(Xl + (row + 8) * kLdX + kt * 16 + 2 * t);
-          const uint32_t hv[4] = {h0[0], h1[0], h0[4], h1[4]};
+          uint32_t d0[4];
 #pragma unroll
-          for (int p = 0; p < 4; ++p) {
-            const __nv_bfloat162 hq = *reinterpret_cast<const __nv_bfloat162*>(&hv[p]);
-            const float* y = &acc[2 * kt + (p >> 1)][2 * (p & 1)];
-            const float m0 = __low2float(hq) > 0.0f ? 1.0f : 0.0f, m1 = __high2float(hq) > 0.0f ? 1.0f : 0.0f;
-            da[kt][p] = pack_bf16(y[0] * m0, y[1] * m1);
-          }
-        }
-        store_a(Dn, row, t, da, 4);
-      } else if (kGrid) {
-        // dX_0 for inputs 0..31 (n-tiles 0..3): acc[nt] holds (row, 8nt+2t+e)
-        // and (row+8, 8nt+2t+e), i.e. level 4nt+t, feature e
-        const bf16* W0 = W + woff(0);
-        float acc[4][4];
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
-#pragma unroll
-        for (int kt = 0; kt < 4; ++kt)
+          for (int p = 0; p < 4; ++p) d0[p] = m ? a[1][kt][p] : a[0][kt][p];
 #pragma unroll
           for (int np = 0; np < 2; ++np) {
-            uint32_t b[4];
-            ldsm_x4(b, W0 + (np * 16 + rr + 8 * (q >> 1)) * ldw(0) + kt * 16 + 8 * (q & 1));
-            mma_bf16(acc[2 * np], da[kt], b[0], b[1]);
-            mma_bf16(acc[2 * np + 1], da[kt], b[2], b[3]);
+            uint32_t b0[4];
+            ldsm_x4(b0, W0 + (np * 16 + rr + 8 * (q >> 1)) * ldw(0) + kt * 16 + 8 * (q & 1));
+            mma_bf16(dx[2 * np], d0, b0[0], b0[1]);
+            mma_bf16(dx[2 * np + 1], d0, b0[2], b0[3]);
           }
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const uint32_t idx = h ? i1 : i0;
+          const uint32_t idx = first + (uint32_t)row + 16u * m + 8u * h;
           if (idx >= count) continue;
           const NrcRecord& rec = recs[idx];
           float ux, uy, uz;
@@ -305,7 +613,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) nrc_train_kernel(NrcView v, 
           for (int nt = 0; nt < 4; ++nt) {
             const int lv = 4 * nt + t;
             if (lv >= v.levels) continue;
-            const float d0 = acc[nt][2 * h], d1 = acc[nt][2 * h + 1];
+            const float d0 = dx[nt][2 * h], d1 = dx[nt][2 * h + 1];
             const int n = nrc_grid_res(lv);
             const NrcGridCell c = nrc_grid_cell(n, ux, uy, uz);
             float* gl = v.ggrad + (size_t)lv * kNrcGridTable * 2;
@@ -320,24 +628,6 @@ __global__ void __launch_bounds__(kTrainThreads, 1) nrc_train_kernel(NrcView v, 
         }
       }
     }
-    __syncthreads();  // every warp is done with X_0 and dY_0 before the next tile's
-  }
-  // the CTA's gradient ([in][out] layout per layer) into its own slot of
-  // gpart, every weight written (the warps' blocks cover each layer once);
-  // nrc_grad_reduce_kernel sums the slots in a fixed order
-  float* slot = gpart + (size_t)blockIdx.x * kNrcWeightCount;
-#pragma unroll
-  for (int l = 0; l < kNrcHidden; ++l)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float* base = slot + nrc_layer_offset(l) + (mt * 16 + g) * kNrcWidth + half * 32 + j * 8 + 2 * t;
-      *reinterpret_cast<float2*>(base) = make_float2(dwh[l][j][0], dwh[l][j][1]);
-      *reinterpret_cast<float2*>(base + 8 * kNrcWidth) = make_float2(dwh[l][j][2], dwh[l][j][3]);
-    }
-  {
-    float* base = slot + nrc_layer_offset(kNrcHidden) + (mt * 16 + g) * kNrcOutPad + half * 8 + 2 * t;
-    *reinterpret_cast<float2*>(base) = make_float2(dwo[0], dwo[1]);
-    *reinterpret_cast<float2*>(base + 8 * kNrcOutPad) = make_float2(dwo[2], dwo[3]);
   }
   for (int o = 16; o > 0; o >>= 1) loss_local += __shfl_xor_sync(0xffffffffu, loss_local, o);
   if (lane == 0) atomicAdd(loss, loss_local);
@@ -377,6 +667,8 @@ __global__ void __launch_bounds__(kReduceCols * kReduceGroups)
                            uint32_t capacity, uint32_t first_rec, float* __restrict__ grad, AdamView a, AdamStep h,
                            float* __restrict__ loss) {
   __shared__ float part[kReduceGroups][kReduceCols];
+  grid_wait();
+  grid_trigger();
   if (blockIdx.x == 0 && threadIdx.x == 0) {  // the step's loss, and a zero sum for the next step
     loss[1] = loss[0];
     loss[0] = 0.0f;
@@ -476,7 +768,7 @@ __global__ void nrc_grid_init_kernel(float* __restrict__ w, float* __restrict__ 
 // ---------------------------------------------------------------------------
 static size_t infer_smem() { return (size_t)kWs * 2 + kNrcPosLevels * 3 * sizeof(float); }
 static size_t train_smem() {
-  return (size_t)kWs * 2 + (size_t)(kNrcLayers + 2) * kTileX * 2 + kNrcPosLevels * 3 * sizeof(float);
+  return (size_t)kWs * 2 + (size_t)(kNrcLayers + 3) * kTileX * 2 + kNrcPosLevels * 3 * sizeof(float);
 }
 
 size_t nrc_param_count(const NrcState* st) {
@@ -597,6 +889,22 @@ vcr_status nrc_setup(vcr_ctx* ctx, const vcr_nrc_params* p) {
   return VCR_OK;
 }
 
+template <class... P, class... A>
+static cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                     A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Gradient of the loss over records [first, first + capacity) of the
 // *d_count written (device): added to grad, or (adam) followed by one Adam
 // step in the same reduction launch.
@@ -604,18 +912,10 @@ static vcr_status nrc_grad(vcr_ctx* ctx, const NrcRecord* recs, const uint32_t* 
                            cudaStream_t s, uint32_t first, bool adam) {
   NrcState* st = ctx->nrc;
   const int blocks = st->gpart_blocks;
-  if (st->gw) {
-    VCR_CUDA(ctx, cudaFuncSetAttribute(nrc_train_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)train_smem()));
-    nrc_train_kernel<true><<<blocks, kTrainThreads, train_smem(), s>>>(nrc_view(ctx), recs, d_count, capacity, first,
-                                                                       st->gpart, st->loss);
-  } else {
-    VCR_CUDA(ctx, cudaFuncSetAttribute(nrc_train_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)train_smem()));
-    nrc_train_kernel<false><<<blocks, kTrainThreads, train_smem(), s>>>(nrc_view(ctx), recs, d_count, capacity,
-                                                                        first, st->gpart, st->loss);
-  }
-  VCR_CUDA(ctx, cudaGetLastError());
+  const auto train = st->gw ? nrc_train_kernel<true> : nrc_train_kernel<false>;
+  VCR_CUDA(ctx, cudaFuncSetAttribute(train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem()));
+  VCR_CUDA(ctx, launch_overlapped(train, dim3(blocks), dim3(kTrainThreads), train_smem(), s, nrc_view(ctx), recs, d_count,
+                                  capacity, first, st->gpart, st->loss));
   AdamView a{st->w, reinterpret_cast<bf16*>(st->wb), st->m, st->v, st->ema, reinterpret_cast<bf16*>(st->wbi)};
   AdamStep h{};
   if (adam) {
@@ -630,13 +930,9 @@ static vcr_status nrc_grad(vcr_ctx* ctx, const NrcRecord* recs, const uint32_t* 
     h.decay = std::min(st->prm.ema_decay, (1.0f + (float)st->step) / (10.0f + (float)st->step));
   }
   const dim3 grid(kNrcWeightCount / kReduceCols), block(kReduceCols * kReduceGroups);
-  if (adam)
-    nrc_grad_reduce_kernel<true><<<grid, block, 0, s>>>(st->gpart, blocks, d_count, capacity, first, st->grad, a, h,
-                                                        st->loss);
-  else
-    nrc_grad_reduce_kernel<false><<<grid, block, 0, s>>>(st->gpart, blocks, d_count, capacity, first, st->grad, a, h,
-                                                         st->loss);
-  VCR_CUDA(ctx, cudaGetLastError());
+  const auto reduce = adam ? nrc_grad_reduce_kernel<true> : nrc_grad_reduce_kernel<false>;
+  VCR_CUDA(ctx, launch_overlapped(reduce, grid, block, 0, s, st->gpart, blocks, d_count, capacity, first, st->grad, a, h,
+                                  st->loss));
   if (adam && st->gw) {
     nrc_grid_adam_kernel<<<ctx->sm_count * 8, 256, 0, s>>>(st->gw, st->gm, st->gv, st->ggrad, st->gema, h);
     VCR_CUDA(ctx, cudaGetLastError());
