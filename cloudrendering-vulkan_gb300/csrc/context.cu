@@ -178,6 +178,7 @@ extern "C" VCR_API vcr_status vcr_destroy(vcr_ctx* ctx) {
   ppm_free(ctx);
   nrc_free(ctx);
   batch_free(ctx);
+  upload_free(ctx);
   if (ctx->work_done) cudaEventDestroy(ctx->work_done);
   for (int i = 0; i < 2; ++i) {
     cudaFree(ctx->rb.stage[i]);

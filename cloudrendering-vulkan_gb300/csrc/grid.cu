@@ -26,11 +26,71 @@ __global__ void fbm_kernel(float* __restrict__ out, uint64_t total) {
   }
 }
 
+// Brick summaries for the majorants: per brick, the maximum decoded texel
+// over each of the 27 sets "x in X, y in Y, z in Z" with each set one of
+// {0} (the low face), {0..7} (the whole brick), {7} (the high face); entry
+// sx + 3 sy + 9 sz with 0 = low face, 1 = whole, 2 = high face.  v: the
+// decoded rows r = lane + 32 h of the warp's brick, r = y + 8 z.  A lane holds
+// one y, so the maxima over y are those of its group of eight lanes and the
+// maxima over z those of the lanes of the same y: 30 shuffles, and four lanes
+// store what they end up with.
+__device__ __forceinline__ void store_summary(const float (&v)[2][8], int lane, float* __restrict__ out) {
+  constexpr unsigned kAll = 0xffffffffu;
+  float row[2][3], group[2][3], column[3], whole[3];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float m = v[h][0];
+#pragma unroll
+    for (int x = 1; x < 8; ++x) m = fmaxf(m, v[h][x]);
+    row[h][0] = v[h][0];
+    row[h][1] = m;
+    row[h][2] = v[h][7];
+#pragma unroll
+    for (int sx = 0; sx < 3; ++sx) {
+      float g = row[h][sx];
+      for (int o = 4; o > 0; o >>= 1) g = fmaxf(g, __shfl_xor_sync(kAll, g, o));
+      group[h][sx] = g;  // all y of the lane's z
+    }
+  }
+#pragma unroll
+  for (int sx = 0; sx < 3; ++sx) {
+    float c = fmaxf(row[0][sx], row[1][sx]), w = fmaxf(group[0][sx], group[1][sx]);
+    for (int o = 16; o > 4; o >>= 1) {
+      c = fmaxf(c, __shfl_xor_sync(kAll, c, o));
+      w = fmaxf(w, __shfl_xor_sync(kAll, w, o));
+    }
+    column[sx] = c;  // all z of the lane's y
+    whole[sx] = w;
+  }
+  const int y = lane & 7, z = lane >> 3;  // z of row lane; row lane + 32 is at z + 4
+#pragma unroll
+  for (int sx = 0; sx < 3; ++sx) {
+    // zero at least, as the grid's outside
+    if (lane == 0) {
+      out[sx + 3 * 0 + 9 * 0] = fmaxf(0.0f, row[0][sx]);
+      out[sx + 3 * 1 + 9 * 0] = fmaxf(0.0f, group[0][sx]);
+      out[sx + 3 * 0 + 9 * 1] = fmaxf(0.0f, column[sx]);
+      out[sx + 3 * 1 + 9 * 1] = fmaxf(0.0f, whole[sx]);
+    }
+    if (y == 7 && z == 0) {
+      out[sx + 3 * 2 + 9 * 0] = fmaxf(0.0f, row[0][sx]);
+      out[sx + 3 * 2 + 9 * 1] = fmaxf(0.0f, column[sx]);
+    }
+    if (y == 0 && z == 3) {
+      out[sx + 3 * 0 + 9 * 2] = fmaxf(0.0f, row[1][sx]);
+      out[sx + 3 * 1 + 9 * 2] = fmaxf(0.0f, group[1][sx]);
+    }
+    if (y == 7 && z == 3) out[sx + 3 * 2 + 9 * 2] = fmaxf(0.0f, row[1][sx]);
+  }
+}
+
 // One warp per brick (8 bricks per 256-thread CTA): lane l holds texel rows
 // l and l + 32 of the brick (row r = y + 8 z, 8 texels along x, zero
 // outside the grid), the warp's maximum is the brick's scale, and each row
 // is stored as one 16-byte (FP16 / BF16) or two (FP32) vectors into the
-// brick's contiguous 512 texels.
+// brick's contiguous 512 texels.  The brick's summary is taken from the texels
+// as they are stored (a pass of its own over the bricks took 47 us of a 256^3
+// upload, after the last copy).
 constexpr int kBrickWarps = 8;
 
 // `dense` holds z planes [8 kb0, ...) of the grid: the whole grid (kb0 = 0)
@@ -40,7 +100,7 @@ __global__ void __launch_bounds__(kBrickWarps * 32) brick_kernel(const float* __
                                                                  void* __restrict__ bricks,
                                                                  float* __restrict__ scales, int nx, int ny, int nz,
                                                                  int bx, int by, uint32_t b0, uint32_t count,
-                                                                 int kb0) {
+                                                                 int kb0, float* __restrict__ summary) {
   const uint32_t local = blockIdx.x * kBrickWarps + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (local >= count) return;  // warp-uniform
@@ -76,6 +136,7 @@ __global__ void __launch_bounds__(kBrickWarps * 32) brick_kernel(const float* __
       dst[0] = make_float4(v[h][0], v[h][1], v[h][2], v[h][3]);
       dst[1] = make_float4(v[h][4], v[h][5], v[h][6], v[h][7]);
     }
+    store_summary(v, lane, summary + (size_t)b * 27);
     return;
   }
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -89,15 +150,20 @@ __global__ void __launch_bounds__(kBrickWarps * 32) brick_kernel(const float* __
       if (P == 1) {
         const __half2 hv = __halves2half2(__float2half_rn(q0), __float2half_rn(q1));
         w[x / 2] = *reinterpret_cast<const uint32_t*>(&hv);
+        v[h][x] = __low2float(hv) * s;
+        v[h][x + 1] = __high2float(hv) * s;
       } else {
         const __nv_bfloat162 bv = __halves2bfloat162(__float2bfloat16_rn(q0), __float2bfloat16_rn(q1));
         w[x / 2] = *reinterpret_cast<const uint32_t*>(&bv);
+        v[h][x] = __low2float(bv) * s;
+        v[h][x + 1] = __high2float(bv) * s;
       }
     }
     uint16_t* base16 = reinterpret_cast<uint16_t*>(bricks) + brick + 8 * (lane + 32 * h);
     *reinterpret_cast<uint4*>(base16) = make_uint4(w[0], w[1], w[2], w[3]);
   }
   if (lane == 0) scales[b] = s;
+  store_summary(v, lane, summary + (size_t)b * 27);
 }
 
 // The stored grid decoded to dense floats, x fastest (texel() per voxel).
@@ -108,56 +174,6 @@ __global__ void decode_kernel(GridView g, float* __restrict__ out, uint64_t tota
     const uint64_t r = idx / nx;
     out[idx] = texel(g, (int)(idx - r * nx), (int)(r % ny), (int)(r / ny));
   }
-}
-
-// Brick summaries for the majorants: per brick, the maximum decoded texel
-// over each of the 27 sets "x in X, y in Y, z in Z" with each set one of
-// {0} (the low face), {0..7} (the whole brick), {7} (the high face); entry
-// sx + 3 sy + 9 sz with 0 = low face, 1 = whole, 2 = high face.  One warp
-// per brick, lane l holding texel rows l and l + 32 (row r = y + 8 z).
-constexpr int kSumWarps = 8;
-
-__global__ void __launch_bounds__(kSumWarps * 32) brick_summary_kernel(GridView g, float* __restrict__ summary,
-                                                                      uint32_t nbricks) {
-  const uint32_t b = blockIdx.x * kSumWarps + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (b >= nbricks) return;  // warp-uniform
-  float m[27];
-#pragma unroll
-  for (int e = 0; e < 27; ++e) m[e] = 0.0f;
-  const float s = g.precision == 0 ? 1.0f : __ldg(g.scales + b);
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int r = lane + 32 * h, y = r & 7, z = r >> 3;
-    float v[8];
-    const size_t off = ((size_t)b << 9) + 8 * (size_t)r;
-#pragma unroll
-    for (int x = 0; x < 8; ++x) {
-      if (g.precision == 0) v[x] = __ldg(reinterpret_cast<const float*>(g.bricks) + off + x);
-      else if (g.precision == 1) v[x] = __half2float(__ldg(reinterpret_cast<const __half*>(g.bricks) + off + x)) * s;
-      else v[x] = __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(g.bricks) + off + x)) * s;
-    }
-    float row = v[0];
-#pragma unroll
-    for (int x = 1; x < 8; ++x) row = fmaxf(row, v[x]);
-    const float sel_x[3] = {v[0], row, v[7]};
-#pragma unroll
-    for (int sz = 0; sz < 3; ++sz) {
-      if (!(sz == 1 || (sz == 0 && z == 0) || (sz == 2 && z == 7))) continue;
-#pragma unroll
-      for (int sy = 0; sy < 3; ++sy) {
-        if (!(sy == 1 || (sy == 0 && y == 0) || (sy == 2 && y == 7))) continue;
-#pragma unroll
-        for (int sx = 0; sx < 3; ++sx) m[sx + 3 * sy + 9 * sz] = fmaxf(m[sx + 3 * sy + 9 * sz], sel_x[sx]);
-      }
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < 27; ++e)
-    for (int o = 16; o > 0; o >>= 1) m[e] = fmaxf(m[e], __shfl_xor_sync(0xffffffffu, m[e], o));
-#pragma unroll
-  for (int e = 0; e < 27; ++e)
-    if (lane == e) summary[(size_t)b * 27 + e] = m[e];
 }
 
 // Brick majorant from the summaries: the texels in [8b-1, 8b+8] per axis
@@ -188,21 +204,42 @@ __global__ void majorant_from_summary_kernel(const float* __restrict__ summary, 
   atomicMax(gmax, __float_as_uint(m));  // non-negative floats order as integers
 }
 
-// Level l+1 of the majorant pyramid: max over the (up to) 2x2x2 cells of
-// level l it covers.
-__global__ void majorant_reduce_kernel(const float* __restrict__ src, int sx, int sy, int sz,
-                                       float* __restrict__ dst, int dx, int dy, int dz) {
-  uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= (uint32_t)(dx * dy * dz)) return;
-  int i = (int)(c % (uint32_t)dx), j = (int)((c / (uint32_t)dx) % (uint32_t)dy), k = (int)(c / ((uint32_t)dx * dy));
-  float m = 0.0f;
-  for (int dk = 0; dk < 2; ++dk)
-    for (int dj = 0; dj < 2; ++dj)
-      for (int di = 0; di < 2; ++di) {
-        int a = 2 * i + di, b = 2 * j + dj, e = 2 * k + dk;
-        if (a < sx && b < sy && e < sz) m = fmaxf(m, src[(size_t)a + (size_t)sx * ((size_t)b + (size_t)sy * e)]);
-      }
-  dst[c] = m;
+// Levels 1..3 of the majorant pyramid, each cell the maximum over the cells
+// of level 0 that it covers (2^l a side, fewer at the grid's end): one launch
+// for levels that one after the other waited for each other's.  A warp takes
+// one cell of level 3: lane l reads the 2 x 8 cells of level 0 under its cells
+// l and l + 32 of level 1 (4^3, x fastest), and the maxima go up by shuffles.
+struct PyramidView {
+  int n[4][3];       // cells per axis
+  size_t offset[4];  // first cell
+};
+__global__ void majorant_pyramid_kernel(float* __restrict__ maj, PyramidView p, uint32_t cells3) {
+  const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= cells3) return;  // warp-uniform
+  const int lane = (int)(threadIdx.x & 31u);
+  const uint32_t dx = (uint32_t)p.n[3][0], dy = (uint32_t)p.n[3][1];
+  const int at3[3] = {(int)(c % dx), (int)((c / dx) % dy), (int)(c / (dx * dy))};
+  auto index = [&](int l, int i, int j, int k) {
+    return p.offset[l] + (size_t)i + (size_t)p.n[l][0] * ((size_t)j + (size_t)p.n[l][1] * (size_t)k);
+  };
+  auto inside = [&](int l, int i, int j, int k) { return i < p.n[l][0] && j < p.n[l][1] && k < p.n[l][2]; };
+  float m3 = 0.0f;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = 4 * at3[0] + (lane & 3), j = 4 * at3[1] + ((lane >> 2) & 3), k = 4 * at3[2] + (lane >> 4) + 2 * h;
+    float m = 0.0f;
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {
+      const int a = 2 * i + (o & 1), b = 2 * j + ((o >> 1) & 1), e = 2 * k + (o >> 2);
+      if (inside(0, a, b, e)) m = fmaxf(m, maj[index(0, a, b, e)]);
+    }
+    if (inside(1, i, j, k)) maj[index(1, i, j, k)] = m;
+    for (int o = 1; o <= 16; o <<= 2) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));  // 2^3: lanes' lowest bits
+    if (!(lane & 21) && inside(2, i >> 1, j >> 1, k >> 1)) maj[index(2, i >> 1, j >> 1, k >> 1)] = m;
+    m3 = fmaxf(m3, m);
+  }
+  for (int o = 2; o <= 8; o <<= 2) m3 = fmaxf(m3, __shfl_xor_sync(0xffffffffu, m3, o));
+  if (lane == 0) maj[index(3, at3[0], at3[1], at3[2])] = m3;
 }
 
 __global__ void sample_kernel(GridView g, SceneView s, const float* __restrict__ pos, float* __restrict__ out,
@@ -402,28 +439,33 @@ static vcr_status grid_alloc(vcr_ctx* ctx, const vcr_grid_desc* desc, int precis
   return VCR_OK;
 }
 
-// Bricks [b0, b0 + count) from `dense`, which holds z planes [8 kb0, ...).
+// The summaries of a grid's bricks at the start of the scratch buffer, and
+// `extra` bytes behind them (ensure_scratch for what follows).
+static size_t summary_bytes(uint64_t nbricks) { return ((size_t)nbricks * 27 * sizeof(float) + 255) & ~(size_t)255; }
+
+// Bricks [b0, b0 + count) and their summaries from `dense`, which holds z
+// planes [8 kb0, ...).
 static vcr_status brick_launch(vcr_ctx* ctx, const float* dense, const vcr_grid_desc* desc, int precision,
                                uint32_t b0, uint32_t count, int kb0, cudaStream_t s) {
   const int n[3] = {(int)desc->size[0], (int)desc->size[1], (int)desc->size[2]};
   const int bx = (n[0] + kBrick - 1) / kBrick, by = (n[1] + kBrick - 1) / kBrick;
   const unsigned blocks = (count + kBrickWarps - 1) / kBrickWarps;
   if (count == 0) return VCR_OK;
+  float* summary = reinterpret_cast<float*>(ctx->d_scratch);
   if (precision == 0)
     brick_kernel<0><<<blocks, kBrickWarps * 32, 0, s>>>(dense, ctx->d_bricks, ctx->d_scales, n[0], n[1], n[2], bx,
-                                                         by, b0, count, kb0);
+                                                         by, b0, count, kb0, summary);
   else if (precision == 1)
     brick_kernel<1><<<blocks, kBrickWarps * 32, 0, s>>>(dense, ctx->d_bricks, ctx->d_scales, n[0], n[1], n[2], bx,
-                                                         by, b0, count, kb0);
+                                                         by, b0, count, kb0, summary);
   else
     brick_kernel<2><<<blocks, kBrickWarps * 32, 0, s>>>(dense, ctx->d_bricks, ctx->d_scales, n[0], n[1], n[2], bx,
-                                                         by, b0, count, kb0);
+                                                         by, b0, count, kb0, summary);
   VCR_CUDA(ctx, cudaGetLastError());
   return VCR_OK;
 }
 
-// Once every brick is written: brick summaries, majorant pyramid, global
-// maximum, and the corner blocks unless the caller built them already
+// Once every brick and summary is written: majorant pyramid, global maximum, and the corner blocks unless the caller built them already
 // (synchronises on s).
 static vcr_status grid_finish(vcr_ctx* ctx, const vcr_grid_desc* desc, int precision, cudaStream_t s,
                               bool corners_built = false) {
@@ -435,24 +477,18 @@ static vcr_status grid_finish(vcr_ctx* ctx, const vcr_grid_desc* desc, int preci
   for (int a = 0; a < 3; ++a) ctx->nb[a] = nb[a];
   unsigned int* d_gmax = reinterpret_cast<unsigned int*>(ctx->d_counters + 5);
   VCR_CUDA(ctx, cudaMemsetAsync(d_gmax, 0, sizeof(unsigned int), s));
-  GridView g = grid_view(ctx);
-  vcr_status ss = ensure_scratch(ctx, nbricks * 27 * sizeof(float));
-  if (ss) return ss;
-  float* summary = reinterpret_cast<float*>(ctx->d_scratch);
-  brick_summary_kernel<<<(unsigned)((nbricks + kSumWarps - 1) / kSumWarps), kSumWarps * 32, 0, s>>>(
-      g, summary, (uint32_t)nbricks);
+  const float* summary = reinterpret_cast<const float*>(ctx->d_scratch);
   majorant_from_summary_kernel<<<(unsigned)((nbricks + 255) / 256), 256, 0, s>>>(summary, nb[0], nb[1], nb[2],
                                                                                 ctx->d_majorants, d_gmax);
   VCR_CUDA(ctx, cudaGetLastError());
-  for (int l = 1; l < 4; ++l) {
-    const int* sdim = ctx->mnb[l - 1];
-    const int* ddim = ctx->mnb[l];
-    uint32_t cnt = (uint32_t)(ddim[0] * ddim[1] * ddim[2]);
-    majorant_reduce_kernel<<<(cnt + 255) / 256, 256, 0, s>>>(ctx->d_majorants + ctx->moff[l - 1], sdim[0], sdim[1],
-                                                              sdim[2], ctx->d_majorants + ctx->moff[l], ddim[0],
-                                                              ddim[1], ddim[2]);
-    VCR_CUDA(ctx, cudaGetLastError());
+  PyramidView pv{};
+  for (int l = 0; l < 4; ++l) {
+    for (int a = 0; a < 3; ++a) pv.n[l][a] = ctx->mnb[l][a];
+    pv.offset[l] = ctx->moff[l];
   }
+  const uint32_t cells3 = (uint32_t)(pv.n[3][0] * pv.n[3][1] * pv.n[3][2]);
+  majorant_pyramid_kernel<<<(cells3 + 3) / 4, 128, 0, s>>>(ctx->d_majorants, pv, cells3);
+  VCR_CUDA(ctx, cudaGetLastError());
   unsigned int gm = 0;
   VCR_CUDA(ctx, cudaMemcpyAsync(&gm, d_gmax, sizeof(gm), cudaMemcpyDeviceToHost, s));
   VCR_CUDA(ctx, cudaStreamSynchronize(s));
@@ -477,37 +513,50 @@ vcr_status grid_build(vcr_ctx* ctx, const float* d_dense, const vcr_grid_desc* d
   if (st) return st;
   uint32_t nbricks = 1;
   for (int a = 0; a < 3; ++a) nbricks *= ((uint32_t)desc->size[a] + kBrick - 1) / kBrick;
-  st = brick_launch(ctx, d_dense, desc, precision, 0u, nbricks, 0, s);
+  st = ensure_scratch(ctx, summary_bytes(nbricks));
+  if (!st) st = brick_launch(ctx, d_dense, desc, precision, 0u, nbricks, 0, s);
   if (st) return st;
   return grid_finish(ctx, desc, precision, s);
 }
 
+void upload_free(vcr_ctx* ctx) {
+  UploadStreams& u = ctx->upload;
+  for (int r = 0; r < UploadStreams::kSlabs; ++r) {
+    if (u.copied[r]) cudaEventDestroy(u.copied[r]);
+    if (u.done[r]) cudaEventDestroy(u.done[r]);
+  }
+  if (u.copy) cudaStreamDestroy(u.copy);
+  if (u.brick) cudaStreamDestroy(u.brick);
+  u = UploadStreams{};
+}
+
 namespace {
-// Streams, events and the slab ring of one streamed upload.
-struct UploadRing {
-  static constexpr int kSlabs = 3;
-  float* buf = nullptr;
-  cudaStream_t copy = nullptr, brick = nullptr;
-  cudaEvent_t copied[kSlabs] = {}, done[kSlabs] = {};
-  ~UploadRing() {
-    if (copy) cudaStreamSynchronize(copy);
-    if (brick) cudaStreamSynchronize(brick);
-    for (int r = 0; r < kSlabs; ++r) {
-      if (copied[r]) cudaEventDestroy(copied[r]);
-      if (done[r]) cudaEventDestroy(done[r]);
-    }
-    if (copy) cudaStreamDestroy(copy);
-    if (brick) cudaStreamDestroy(brick);
-    cudaFree(buf);
+// Ends the work of an upload that is left early, and a ring of its own.
+struct UploadGuard {
+  UploadStreams& u;
+  float* own = nullptr;
+  ~UploadGuard() {
+    if (u.copy) cudaStreamSynchronize(u.copy);
+    if (u.brick) cudaStreamSynchronize(u.brick);
+    cudaFree(own);
   }
 };
+// A slab holds as many brick layers as make 8 MB: at one layer of a 256^3 grid
+// (2 MB) the two launches a layer took 14 us, the copy 10; slabs of 4, 8 and
+// 16 MB give a 256^3 binding of 542, 476 and 479 us.  Rings up to 64 MB
+// live in the scratch buffer, which the context keeps; larger ones are
+// allocated by the call.
+constexpr size_t kSlabBytes = 8u << 20, kKeptRing = 64u << 20;
 }  // namespace
 
-// A host grid uploaded one brick layer (8 z planes) at a time through a
-// ring of three device slabs: the copy of layer k overlaps the bricking of
-// layer k - 1 and the corner blocks of tile layer k - 1 (which read brick
-// layers k - 2 and k - 1), and no device copy of the whole dense grid is
-// made.
+// A host grid uploaded a slab of brick layers (8 z planes each) at a time
+// through a ring of three device slabs: the copy of a slab overlaps the
+// bricking of the slab before and the corner blocks of its tile layers (tile
+// layer k reads brick layers k - 1 and k), and no device copy of the whole
+// dense grid is made.  The copies bound it (256^3: 332 us of the link); the
+// majorants come on the copies' stream, beside the last corner blocks.  A 256^3
+// upload: 880 us with a slab a layer and streams, events and ring made by every
+// call, 424 so.
 vcr_status grid_upload_host(vcr_ctx* ctx, const float* host, const vcr_grid_desc* desc, int precision) {
   vcr_status st = grid_alloc(ctx, desc, precision, 0);
   if (st) return st;
@@ -517,36 +566,54 @@ vcr_status grid_upload_host(vcr_ctx* ctx, const float* host, const vcr_grid_desc
   const int layers = (int)((nz + kBrick - 1) / kBrick);
   const bool corners = ctx->tuning.corner_blocks != 0;
   if (corners) corner_alloc(ctx);
-  UploadRing ring;
-  VCR_CUDA(ctx, cudaMalloc(&ring.buf, (size_t)UploadRing::kSlabs * kBrick * plane * sizeof(float)));
-  VCR_CUDA(ctx, cudaStreamCreateWithFlags(&ring.copy, cudaStreamNonBlocking));
-  VCR_CUDA(ctx, cudaStreamCreateWithFlags(&ring.brick, cudaStreamNonBlocking));
-  for (int r = 0; r < UploadRing::kSlabs; ++r) {
-    VCR_CUDA(ctx, cudaEventCreateWithFlags(&ring.copied[r], cudaEventDisableTiming));
-    VCR_CUDA(ctx, cudaEventCreateWithFlags(&ring.done[r], cudaEventDisableTiming));
+  UploadStreams& u = ctx->upload;
+  constexpr int kSlabs = UploadStreams::kSlabs;
+  const size_t layer = kBrick * plane;  // floats
+  const int per = (int)std::max<size_t>(1, std::min<size_t>((size_t)layers, kSlabBytes / (layer * sizeof(float))));
+  const size_t ring = (size_t)std::min(kSlabs, (layers + per - 1) / per) * per * layer * sizeof(float);
+  const size_t head = summary_bytes((uint64_t)bx * by * layers);
+  UploadGuard guard{u};
+  st = ensure_scratch(ctx, head + (ring <= kKeptRing ? ring : 0));
+  if (st) return st;
+  float* slabs = reinterpret_cast<float*>(reinterpret_cast<char*>(ctx->d_scratch) + head);
+  if (ring > kKeptRing) {
+    VCR_CUDA(ctx, cudaMalloc(&guard.own, ring));
+    slabs = guard.own;
   }
-  for (int kb = 0; kb < layers; ++kb) {
-    const int r = kb % UploadRing::kSlabs;
-    float* slab = ring.buf + (size_t)r * kBrick * plane;
-    if (kb >= UploadRing::kSlabs) VCR_CUDA(ctx, cudaStreamWaitEvent(ring.copy, ring.done[r], 0));
-    const size_t z0 = (size_t)kb * kBrick, planes = std::min<size_t>(kBrick, nz - z0);
+  if (!u.copy) VCR_CUDA(ctx, cudaStreamCreateWithFlags(&u.copy, cudaStreamNonBlocking));
+  if (!u.brick) VCR_CUDA(ctx, cudaStreamCreateWithFlags(&u.brick, cudaStreamNonBlocking));
+  for (int r = 0; r < kSlabs; ++r) {
+    if (!u.copied[r]) VCR_CUDA(ctx, cudaEventCreateWithFlags(&u.copied[r], cudaEventDisableTiming));
+    if (!u.done[r]) VCR_CUDA(ctx, cudaEventCreateWithFlags(&u.done[r], cudaEventDisableTiming));
+  }
+  int r = 0;
+  for (int kb = 0, slab_index = 0; kb < layers; kb += per, ++slab_index) {
+    r = slab_index % kSlabs;
+    float* slab = slabs + (size_t)r * per * layer;
+    if (slab_index >= kSlabs) VCR_CUDA(ctx, cudaStreamWaitEvent(u.copy, u.done[r], 0));
+    const int count = std::min(per, layers - kb);
+    const size_t z0 = (size_t)kb * kBrick, planes = std::min<size_t>((size_t)count * kBrick, nz - z0);
     VCR_CUDA(ctx, cudaMemcpyAsync(slab, host + z0 * plane, planes * plane * sizeof(float), cudaMemcpyHostToDevice,
-                                  ring.copy));
-    VCR_CUDA(ctx, cudaEventRecord(ring.copied[r], ring.copy));
-    VCR_CUDA(ctx, cudaStreamWaitEvent(ring.brick, ring.copied[r], 0));
-    st = brick_launch(ctx, slab, desc, precision, (uint32_t)kb * bx * by, bx * by, kb, ring.brick);
+                                  u.copy));
+    VCR_CUDA(ctx, cudaEventRecord(u.copied[r], u.copy));
+    VCR_CUDA(ctx, cudaStreamWaitEvent(u.brick, u.copied[r], 0));
+    st = brick_launch(ctx, slab, desc, precision, (uint32_t)kb * bx * by, (uint32_t)count * bx * by, kb, u.brick);
     if (st) return st;
-    VCR_CUDA(ctx, cudaEventRecord(ring.done[r], ring.brick));
+    VCR_CUDA(ctx, cudaEventRecord(u.done[r], u.brick));
     if (corners) {
-      st = corner_layers(ctx, (uint32_t)kb, (uint32_t)kb + 1u, ring.brick);
+      st = corner_layers(ctx, (uint32_t)kb, (uint32_t)(kb + count), u.brick);
       if (st) return st;
     }
   }
   if (corners) {  // the tile layer past the last brick layer (clamped texels)
-    st = corner_layers(ctx, (uint32_t)layers, (uint32_t)ctx->corner_tiles[2], ring.brick);
+    st = corner_layers(ctx, (uint32_t)layers, (uint32_t)ctx->corner_tiles[2], u.brick);
     if (st) return st;
   }
-  return grid_finish(ctx, desc, precision, ring.brick, corners);
+  VCR_CUDA(ctx, cudaStreamWaitEvent(u.copy, u.done[r], 0));  // every brick and summary
+  st = grid_finish(ctx, desc, precision, u.copy, corners);
+  if (st) return st;
+  VCR_CUDA(ctx, cudaStreamSynchronize(u.brick));  // the corner blocks
+  return VCR_OK;
 }
 
 vcr_status grid_sample_launch(vcr_ctx* ctx, const float* d_pos, float* d_out, uint32_t n, cudaStream_t s) {

@@ -18,6 +18,15 @@ struct NrcState;
 struct BatchState;
 }  // namespace vcr
 
+namespace vcr {
+// Streams and events of grid uploads from host memory (made by the first).
+struct UploadStreams {
+  static constexpr int kSlabs = 3;  // slabs of the ring
+  cudaStream_t copy = nullptr, brick = nullptr;
+  cudaEvent_t copied[kSlabs] = {}, done[kSlabs] = {};
+};
+}  // namespace vcr
+
 struct vcr_ctx {
   int device = 0;
   int sm_count = 0;
@@ -66,6 +75,8 @@ struct vcr_ctx {
     size_t bytes = 0;
     int slot = 0;
   } rb;
+
+  vcr::UploadStreams upload;
 
   // device counters: [0] paths [1] lookups [2] events [3] dda cells [4] work cursor
   // [5] grid max (u32 bits) [6] training-path cursor [7] relRMSE accumulator (double bits)
@@ -137,6 +148,7 @@ SceneView scene_view(const vcr_ctx* ctx);
 // grid.cu
 // A host grid, uploaded and bricked one brick layer at a time.
 vcr_status grid_upload_host(vcr_ctx* ctx, const float* host, const vcr_grid_desc* desc, int precision);
+void upload_free(vcr_ctx* ctx);
 vcr_status grid_build(vcr_ctx* ctx, const float* d_dense, const vcr_grid_desc* desc, int precision,
                       cudaStream_t s);
 // The corner blocks of the bound grid (after the bricks are written).
