@@ -604,6 +604,69 @@ __device__ __forceinline__ uint32_t tile_pixels(const TileView& t, float4 lo, fl
   return row * ((kRows << (kW * ya)) & (kRows >> (kW * (kH - 1u - yb))));
 }
 
+// The pixels of the tile whose rays can come within r of the segment (start
+// pa, unit direction bd, length segl) at a point between its ends: the pixels
+// beam_closest can pass, and few others.  With the ray of pixel (a, b) from
+// the apex along q = Q + a R + b U (not normalised) and w the apex relative to
+// an end of the segment, the two lines are |q . (bd x w)| / |q x bd| apart,
+// and their closest points lie past that end of the segment, along bd, where
+// (q x w) . (q x bd) > 0.  The first is linear in (a, b) with the right-hand
+// side bounded over the tile; the second is quadratic, its linear part at the
+// tile's centre and a bound of the rest are used.  Margins over the rounding
+// here and in beam_closest: there t and sb are off by some 1e-6 |w| / den,
+// which is 1e-6 |w| |q|^2 of (q x w) . (q x bd) whatever den is (2e-5 allowed);
+// distances by 1e-7 of the coordinates (grow: 1e-5).  A form that is not
+// finite leaves the pixel in.
+//
+// A segment is about as long as its radius, so its box covers five times the
+// pixels that pass.  1280x720, 60,741 photons: 2.31 G (leaf, pixel) pairs of
+// the boxes' ranges become 0.64 G, of which 0.44 G pass; gather 25.1 -> 20.6 ms.
+__device__ __forceinline__ float sum_abs(f3 v) { return (fabsf(v.x) + fabsf(v.y)) + fabsf(v.z); }
+__device__ __forceinline__ f3 fcross(f3 a, f3 b) {
+  return mk(fmaf(a.y, b.z, -(a.z * b.y)), fmaf(a.z, b.x, -(a.x * b.z)), fmaf(a.x, b.y, -(a.y * b.x)));
+}
+__device__ __forceinline__ float fdot(f3 a, f3 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, a.z * b.z)); }
+template <uint32_t kW, uint32_t kH>
+__device__ __forceinline__ uint32_t near_pixels(const CamView& cam, float grow, int x0, int y0, f3 pa, float r, f3 bd,
+                                                float segl) {
+  constexpr float hx = 0.5f * (float)(kW - 1u), hy = 0.5f * (float)(kH - 1u);
+  const f3 R = cam.right * cam.px, U = -(cam.up * cam.py);
+  const f3 Q = cam.fwd * cam.near_plane + R * ((float)(x0 - cam.hw) + hx) + U * ((float)(y0 - cam.hh) + hy);
+  const f3 w = cam.pos - pa;
+  const float qn = sum_abs(Q) + hx * sum_abs(R) + hy * sum_abs(U), wn = sum_abs(w) + segl;
+  const f3 c = fcross(Q, bd), cR = fcross(R, bd), cU = fcross(U, bd), m = fcross(bd, w);
+  const float dc = hx * sum_abs(cR) + hy * sum_abs(cU);  // q x bd is within this of c
+  // |f| <= F
+  const float fR = fdot(R, m), fU = fdot(U, m);
+  const float F = fmaf(fmaf(r, 1.0001f, grow), fmaf(sqrtf(fdot(c, c)), 1.0001f, dc), 4e-6f * (qn * wn));
+  // g0 >= -G0 at the start, g1 <= G1 at the end (w - segl bd)
+  const f3 e = fcross(Q, w), eR = fcross(R, w), eU = fcross(U, w);
+  const float g0R = fdot(eR, c) + fdot(e, cR), g0U = fdot(eU, c) + fdot(e, cU);
+  const float round = (qn * qn) * fmaf(2e-5f, wn, grow);
+  const float G0 = fmaf(1.01f * (hx * sum_abs(eR) + hy * sum_abs(eU)), dc, round);
+  const float G1 = fmaf(1.01f * segl * dc, dc, G0);
+  const float cc = fdot(c, c), g1R = fmaf(-2.0f * segl, fdot(c, cR), g0R), g1U = fmaf(-2.0f * segl, fdot(c, cU), g0U);
+  float f = fmaf(-hx, fR, fmaf(-hy, fU, fdot(Q, m)));
+  float g0 = fmaf(-hx, g0R, fmaf(-hy, g0U, fdot(e, c)));
+  float g1 = fmaf(-hx, g1R, fmaf(-hy, g1U, fmaf(-segl, cc, fdot(e, c))));
+  uint32_t pixels = 0;
+#pragma unroll
+  for (uint32_t y = 0; y < kH; ++y) {
+    float a = f, b = g0, d = g1;
+#pragma unroll
+    for (uint32_t x = 0; x < kW; ++x) {
+      if (!(fabsf(a) > F || b < -G0 || d > G1)) pixels |= 1u << (y * kW + x);
+      a += fR;
+      b += g0R;
+      d += g1R;
+    }
+    f += fU;
+    g0 += g0U;
+    g1 += g1U;
+  }
+  return pixels;
+}
+
 // Beam x beam (1D) estimate of one segment (accumulateRadiance,
 // PPB_PE.comp:362-404, with the fixes named at the top of the file), in two
 // steps.  The first, for every (ray, segment) pair: the closest points of
@@ -611,9 +674,13 @@ __device__ __forceinline__ uint32_t tile_pixels(const TileView& t, float4 lo, fl
 // length segl), at t along the ray and sb along the segment; false where the
 // pair contributes nothing.  The distance is compared squared, with a margin
 // over the rounding of the square root; the second step decides with it.
-__device__ __forceinline__ bool beam_closest(f3 pa, float r, f3 bd, float segl, f3 o, f3 rd, float t_in, float t_far,
-                                             float& t, float& sb) {
-  if (!(segl > 0.0f)) return false;
+// (A segment of no length has no direction: the caller leaves it out.)
+__device__ __forceinline__ float closest_limit(float r) {
+  const float r2 = r * r;
+  return r2 > 1e-30f ? r2 * 1.000001f : INFINITY;
+}
+__device__ __forceinline__ bool beam_closest(f3 pa, float limit, f3 bd, float segl, f3 o, f3 rd, float t_in,
+                                             float t_far, float& t, float& sb) {
   float b = dot(rd, bd);
   float den = 1.0f - b * b;
   if (!(den > 1e-6f)) return false;  // (nearly) parallel
@@ -623,8 +690,7 @@ __device__ __forceinline__ bool beam_closest(f3 pa, float r, f3 bd, float segl, 
   sb = ew + t * b;
   if (t < t_in || t > t_far || sb < 0.0f || sb > segl) return false;
   const f3 e = along(o, rd, t) - along(pa, bd, sb);
-  const float r2 = r * r;
-  return dot(e, e) < r2 * 1.000001f || !(r2 > 1e-30f);
+  return dot(e, e) < limit;
 }
 
 // The second step: the contribution of a pair the first one kept.  off: the
@@ -657,9 +723,10 @@ __device__ __forceinline__ f3 beam_contribution(const GridView& g, const SceneVi
   float tc = t - t_in;
   uint32_t below = 0;  // camera flights shorter than tc
 #pragma unroll
-  for (uint32_t k = 8; k > 0; k >>= 1)
-    if (__ldg(dist16 + below + k - 1) < tc) below += k;
-  if (below == 15u && __ldg(dist16 + 15) < tc) below = 16u;
+  for (int i = 0; i < kBeamDists / 4; ++i) {
+    const float4 q = __ldg(reinterpret_cast<const float4*>(dist16) + i);
+    below += (q.x < tc ? 1u : 0u) + (q.y < tc ? 1u : 0u) + (q.z < tc ? 1u : 0u) + (q.w < tc ? 1u : 0u);
+  }
   uint32_t cc = (uint32_t)kBeamDists - below;
   float tb = (float)cb * (1.0f / kBeamDists), tcam = (float)cc * (1.0f / kBeamDists);
   float ph = hg_pdf(s.ph, dot(bd, -rd));
@@ -670,24 +737,26 @@ __device__ __forceinline__ f3 beam_contribution(const GridView& g, const SceneVi
 // Per-pixel gather.  A warp takes a tile of P pixels and finds the leaves
 // whose boxes its rays may meet by descending the 32-wide cluster boxes, one
 // lane a box (coalesced loads; the box's pixel range in the tile by three
-// linear forms).  The kept leaves' segments go to shared memory with their
-// directions and lengths worked out once a tile and the pixels they may
-// cover.  The (leaf, pixel) pairs of a batch are listed and tested 32 at a
-// time, one lane a pair: the exact box test (the single-ray walk of the LBVH
-// visits exactly the leaves whose boxes the ray meets, since a ray that
-// meets a box meets every box around it), and the closest points.  The pairs
-// that contribute - about one box hit in five - are queued and evaluated 32
-// at a time, again one lane a pair.  A pixel adds its pairs' contributions
-// in queue order, which is ascending leaf order: the order of the
-// depth-first walk, so the sums are the same floats.
+// linear forms).  The leaves it finds are queued and taken 32 at a time, one
+// lane a leaf, for the direction and length of the segment and the pixels it
+// can contribute to (near_pixels).  The (leaf, pixel) pairs of a batch are
+// listed and tested 32 at a time, one lane a pair, for the closest points;
+// those that pass are queued and evaluated 32 at a time, again one lane a
+// pair, if the ray meets the leaf's box (the single-ray walk of the LBVH
+// visits exactly the leaves whose boxes the ray meets, since a ray that meets
+// a box meets every box around it).  A pixel adds its pairs' contributions in
+// queue order, which is ascending leaf order: the order of the depth-first
+// walk, so the sums are the same floats.
 //
-// Bound by instruction issue (0.75 of the slots at 24 warps an SM), most of
-// it the evaluation's divisions, square roots and gathers.  1280x720, 60,741
-// photons, 9.6 M segments of radius 0.015: 27.5 ms for 1.82 G box hits, of
-// 5.48 G before the leaves and ray ends that give exactly 0 were left out
-// (ppb_live_kernel, t_far; 71.9 ms).  The same walk with one lane a pixel
-// for the closest points and the evaluation, 12 lanes of 32 at work, took
-// 129 ms.
+// Bound by the evaluation's instructions (divisions, square roots, gathers:
+// half of all) and by what the L1 holds beside the warps' shared memory: the
+// leaf slots keep only what the pair test reads (2 KB a warp instead of 4:
+// 21.3 -> 19.9 ms with the camera's kernel; queuing the pairs' distances as
+// well, 0.5 KB more, took 1.7 ms).  1280x720, 60,741 photons, 9.6 M segments of
+// radius 0.015: 18.8 ms for 0.64 G pairs; 27.5 with a box test of each of 2.3 G
+// pairs before the closest points; 71.9 with the leaves and ray ends that give
+// exactly 0 (ppb_live_kernel, t_far); 129 with one lane a pixel for the closest
+// points and the evaluation, 12 lanes of 32 at work.
 constexpr int kGatherThreads = 128;
 constexpr int kGatherWarps = kGatherThreads / 32;
 constexpr int kLeafBatch = 64;  // leaf slots of a warp; a batch is tested once more than 32 are filled
@@ -695,13 +764,14 @@ __host__ __device__ constexpr uint32_t gather_w(int P) { return P == 32 ? 8u : P
 
 template <int P>
 struct __align__(16) GatherWarp {
-  float4 leaf[kLeafBatch][4];  // (box lo, offset) (box hi, beam) (start, radius) (direction, length)
+  float4 leaf[kLeafBatch][2];  // (start, number of the leaf) (direction, length)
   float4 ray[P][3];            // (origin, t_in) (direction, t_far) (1 / direction, t_box)
   float2 q_t[64];              // queued pairs: (t, sb)
   uint32_t q_id[64];           // leaf slot << 5 | pixel
   uint32_t pixels[kLeafBatch]; // the tile's pixels a leaf's box may cover
   float c[3][32];              // contributions of a group of pairs
   uint32_t own[P];             // each pixel's pairs in the group
+  uint2 cand[64];              // leaves whose boxes the tile meets: leaf, pixels of the box
   uint32_t mask[kClusterLevels], base[kClusterLevels];
   uint16_t pair[32 * P];       // the pairs of 32 leaves: leaf slot << 5 | pixel
 };
@@ -728,6 +798,7 @@ __global__ void __launch_bounds__(kGatherThreads, 6) ppb_gather_kernel(const __g
   bool trav = false;
   float depth = -INFINITY;  // W of the tile's farthest ray end
   const uint32_t n = *v.n_live;
+  const float limit = closest_limit(v.radius);  // every segment's radius
   TileView view = tile_view(cam, s, (int)(pv.x0 + tx0), (int)(pv.y0 + ty0), (int)kW, (int)kH);
   if (valid) {
     f3 o, rd;
@@ -766,7 +837,7 @@ __global__ void __launch_bounds__(kGatherThreads, 6) ppb_gather_kernel(const __g
     view.far = depth;
     const int top = v.cl.levels - 1;
     int lev = top;  // warp-uniform, as are filled and the masks
-    uint32_t filled = 0;
+    uint32_t filled = 0, ch = 0, cn = 0;  // leaf slots; first candidate and their number
     bool done = false;
     {
       bool see = false;
@@ -782,7 +853,39 @@ __global__ void __launch_bounds__(kGatherThreads, 6) ppb_gather_kernel(const __g
     }
     while (true) {
       // ---- descend until more than 32 leaves are at hand ----------------
-      while (filled <= 32u && !done) {
+      while (filled <= 32u && !(done && cn == 0u)) {
+        if (cn >= 32u || done) {  // 32 candidates, a lane each: the segment's own pixels
+          const uint32_t take = min(cn, 32u);
+          float4 A = make_float4(0.f, 0.f, 0.f, 0.f), B = A;
+          f3 ax = mk(0.f, 0.f, 0.f);
+          float segl = 0.0f;
+          uint32_t leaf = 0, covers = 0;
+          if (lane < take) {
+            const uint2 q = w.cand[(ch + lane) & 63u];
+            leaf = q.x;
+            A = v.leaf.a[leaf];
+            B = v.leaf.b[leaf];
+            ax = mk(B.x, B.y, B.z) - mk(A.x, A.y, A.z);
+            segl = length(ax);
+            ax = mk(ax.x / segl, ax.y / segl, ax.z / segl);
+            covers = q.y & near_pixels<kW, kH>(cam, view.grow, (int)(pv.x0 + tx0), (int)(pv.y0 + ty0),
+                                               mk(A.x, A.y, A.z), v.radius, ax, segl);
+            if (!(segl > 0.0f)) covers = 0u;
+          }
+          const uint32_t cm = __ballot_sync(0xffffffffu, covers != 0u);
+          if (covers) {
+            const uint32_t at = filled + __popc(cm & lt);
+            float4* f = w.leaf[at];
+            f[0] = make_float4(A.x, A.y, A.z, __uint_as_float(leaf));
+            f[1] = make_float4(ax.x, ax.y, ax.z, segl);
+            w.pixels[at] = covers;
+          }
+          filled += __popc(cm);
+          ch += take;
+          cn -= take;
+          __syncwarp();
+          continue;
+        }
         const uint32_t m = w.mask[lev];
         const uint32_t node = w.base[lev] + __ffs(m) - 1u;
         __syncwarp();
@@ -805,28 +908,11 @@ __global__ void __launch_bounds__(kGatherThreads, 6) ppb_gather_kernel(const __g
             w.base[lev] = node * 32u;
           }
         } else {
-          float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
           uint32_t covers = 0u;
-          if (child < n) {
-            lo = v.leaf.lo[child];
-            hi = v.leaf.hi[child];
-            covers = rays & tile_pixels<kW, kH>(view, lo, hi);
-          }
+          if (child < n) covers = rays & tile_pixels<kW, kH>(view, v.leaf.lo[child], v.leaf.hi[child]);
           const uint32_t cm = __ballot_sync(0xffffffffu, covers != 0u);
-          if (covers) {
-            const float4 A = v.leaf.a[child], B = v.leaf.b[child];
-            const uint32_t beam = v.leaf.beam[child];
-            const f3 ax = mk(B.x, B.y, B.z) - mk(A.x, A.y, A.z);
-            const float segl = length(ax);
-            const uint32_t at = filled + __popc(cm & lt);
-            float4* f = w.leaf[at];
-            f[0] = make_float4(lo.x, lo.y, lo.z, B.w);
-            f[1] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(beam));
-            f[2] = A;
-            f[3] = make_float4(ax.x / segl, ax.y / segl, ax.z / segl, segl);
-            w.pixels[at] = covers;
-          }
-          filled += __popc(cm);
+          if (covers) w.cand[(ch + cn + __popc(cm & lt)) & 63u] = make_uint2(child, covers);
+          cn += __popc(cm);
         }
         __syncwarp();
       }
@@ -843,6 +929,7 @@ __global__ void __launch_bounds__(kGatherThreads, 6) ppb_gather_kernel(const __g
         }
         const uint32_t pairs = __shfl_sync(0xffffffffu, at, 31);
         at -= __popc(pm);
+        segs += __popc(pm);
         for (; pm; pm &= pm - 1u) w.pair[at++] = (uint16_t)(((half + lane) << 5) | (__ffs(pm) - 1u));
         __syncwarp();
         for (uint32_t i = 0; i < pairs; i += 32u) {
@@ -851,16 +938,10 @@ __global__ void __launch_bounds__(kGatherThreads, 6) ppb_gather_kernel(const __g
           uint32_t id = 0;
           if (i + lane < pairs) {
             id = w.pair[i + lane];
-            const float4* f = w.leaf[id >> 5];
-            const float4* q = w.ray[id & 31u];
-            const float4 r0 = q[0], r1 = q[1], r2 = q[2];
-            const f3 o = mk(r0.x, r0.y, r0.z);
-            if (ray_box(o, mk(r2.x, r2.y, r2.z), r0.w, r2.w, f[0], f[1])) {
-              ++segs;
-              const float4 a = f[2], d = f[3];
-              pass = beam_closest(mk(a.x, a.y, a.z), a.w, mk(d.x, d.y, d.z), d.w, o, mk(r1.x, r1.y, r1.z), r0.w, r1.w,
-                                  t, sb);
-            }
+            const float4 r0 = w.ray[id & 31u][0], r1 = w.ray[id & 31u][1];
+            const float4 a = w.leaf[id >> 5][0], d = w.leaf[id >> 5][1];
+            pass = beam_closest(mk(a.x, a.y, a.z), limit, mk(d.x, d.y, d.z), d.w, mk(r0.x, r0.y, r0.z),
+                                mk(r1.x, r1.y, r1.z), r0.w, r1.w, t, sb);
           }
           const uint32_t acc = __ballot_sync(0xffffffffu, pass);
           if (pass) {
@@ -882,12 +963,20 @@ __global__ void __launch_bounds__(kGatherThreads, 6) ppb_gather_kernel(const __g
               const float2 ts = w.q_t[k];
               key = e & 31u;
               const float4* f = w.leaf[e >> 5];
-              const float4 a = f[2], d = f[3], r0 = w.ray[key][0], r1 = w.ray[key][1];
-              const uint32_t beam = __float_as_uint(f[1].w);
-              const uint32_t pixel = (ty0 + key / kW) * pv.cw + tx0 + key % kW;
-              c = beam_contribution(g, s, v.slots + (size_t)beam * kSlotFloats, mk(a.x, a.y, a.z), a.w,
-                                    mk(d.x, d.y, d.z), f[0].w, mk(r0.x, r0.y, r0.z), mk(r1.x, r1.y, r1.z), r0.w, ts.x,
-                                    ts.y, v.cam_dist + (size_t)pixel * kBeamDists, lookups);
+              const float4 a = f[0], d = f[1];
+              const uint32_t leaf = __float_as_uint(a.w), beam = v.leaf.beam[leaf];
+              const float4 lo = v.leaf.lo[leaf], hi = v.leaf.hi[leaf];
+              const float off = v.leaf.b[leaf].w;
+              const float4 r0 = w.ray[key][0], r1 = w.ray[key][1], r2 = w.ray[key][2];
+              const f3 o = mk(r0.x, r0.y, r0.z);
+              if (ray_box(o, mk(r2.x, r2.y, r2.z), r0.w, r2.w, lo, hi)) {
+                const uint32_t pixel = (ty0 + key / kW) * pv.cw + tx0 + key % kW;
+                c = beam_contribution(g, s, v.slots + (size_t)beam * kSlotFloats, mk(a.x, a.y, a.z), v.radius,
+                                      mk(d.x, d.y, d.z), off, o, mk(r1.x, r1.y, r1.z), r0.w, ts.x, ts.y,
+                                      v.cam_dist + (size_t)pixel * kBeamDists, lookups);
+              } else {
+                key = 32u + lane;  // no pair after all
+              }
             }
             const uint32_t peers = __match_any_sync(0xffffffffu, key);
             if (lane < m && (peers & lt) == 0u) w.own[key] = peers;
@@ -908,7 +997,7 @@ __global__ void __launch_bounds__(kGatherThreads, 6) ppb_gather_kernel(const __g
         __syncwarp();
       }
       filled = 0;
-      if (done) break;
+      if (done && cn == 0u) break;
     }
   }
   if (valid) write_result(pv, sum, (pv.y0 + cy) * pv.width + pv.x0 + cx, L);
@@ -933,10 +1022,10 @@ static vcr_status gather_launch_t(vcr_ctx* ctx, const GridView& g, const SceneVi
 // The largest tile that still gives the SMs 84 tiles each, three and a half
 // rounds of the 24 warps an SM holds: a larger tile shares a leaf's set-up
 // among more pixels, a smaller one leaves less work to the longest warp.
-// Measured (gather ms at 32 / 16 / 8 / 4 / 2 pixels a tile, 256^3 cloud):
-// 1280x720, 9.6 M segments 29.1 / 29.3 / 36.3 / 49.0 / -; 640x360, 3.1 M
-// segments 4.98 / 4.40 / 4.57 / 5.72 / -; 320x180 5.11 / 3.31 / 2.41 / 2.36 /
-// -; 160x90 6.20 / 3.91 / 2.61 / 1.89 / 1.61.
+// Measured (ms with the camera's kernel, 256^3 cloud, twice and half that
+// many tiles): 1280x720, 9.6 M segments 20.0 at 32 pixels, 21.0 at 16; 640x360,
+// 3.1 M segments 3.57 / 3.27 / 4.46 at 32 / 16 / 8; 320x180 2.56 / 1.89 / 2.27
+// at 16 / 8 / 4; 160x90 1.55 / 1.30 / 1.30 at 8 / 4 / 2.
 static vcr_status gather_launch(vcr_ctx* ctx, const GridView& g, const SceneView& s, const CamView& cam,
                                 const PassView& pv, const PpbGatherView& gv, Counters cnt,
                                 unsigned long long* d_count, cudaStream_t st) {

@@ -588,10 +588,11 @@ VCR_API vcr_status vcr_ppb_free(vcr_ctx* ctx);
 VCR_API vcr_status vcr_ppb_pass(vcr_ctx* ctx, const vcr_pass_desc* pass, void* stream);
 VCR_API vcr_status vcr_ppb_info(vcr_ctx* ctx, vcr_ppb_info_t* out);
 /* The last pass's gather: (pixel, beam segment) pairs it evaluated (segments
- * whose box the pixel's ray hit, without those that contribute exactly 0:
- * past the beam's or the camera ray's farthest transmittance sample, or in
- * cells without density) and its device time.  Waits for the gather to
- * finish.  No reference counterpart (measurement). */
+ * of which a point may come within the radius of the pixel's ray, without
+ * those that contribute exactly 0: past the beam's or the camera ray's
+ * farthest transmittance sample, or in cells without density) and its device
+ * time.  Waits for the gather to finish.  No reference counterpart
+ * (measurement). */
 VCR_API vcr_status vcr_ppb_gather_stats(vcr_ctx* ctx, uint64_t* segments_evaluated, float* ms);
 /* Synchronous copy of one of the last pass's beam buffers. */
 VCR_API vcr_status vcr_ppb_read(vcr_ctx* ctx, vcr_ppb_buffer which, void* host_out, size_t bytes);

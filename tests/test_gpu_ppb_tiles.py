@@ -69,3 +69,28 @@ def test_camera_poses_match_the_oracle(cuda, pos, fwd):
     want, _ = orc.ppb_pass(g, cloud, cam, prm, 300, 1 << 16, 0.05, 0.8, W, H, seed=5, pass_index=0)
     np.testing.assert_array_equal(got, want)
     assert (want > 0.0).any()
+
+
+# the pixels of a segment's own range: the sun along the view (rays nearly parallel to the beams), across it along an
+# axis (segment ends on planes of rays), thin and thick beams, every tile shape's rounding far off the axis
+@pytest.mark.parametrize("radius", [0.004, 0.11])
+@pytest.mark.parametrize("sun", [(0.0, 0.0, 1.0), (0.0, -1.0, 0.0), (1.0, 0.0, 0.0), (0.6, 0.0, 0.8)])
+def test_segment_ranges_match_the_oracle(cuda, sun, radius):
+    W, H = 71, 43
+    cam = vcr.camera_look((0.0, 0.0, -0.4), (0.0, 0.0, 1.0), 100.0, 0.1, W, H)
+    ctx, g, cloud, cam, prm = _context(W, H, cam)
+    for i in range(3):
+        prm.sun_dir[i] = sun[i]
+    with ctx:
+        ctx.set_params(prm)
+        ctx.ppb_setup(300, 1 << 17, radius, 0.8)
+        ctx.ppb_pass(seed=8, pass_index=0)
+        got = ctx.image_sum()
+        for crop in ((3, 2, 8, 4), (W - 9, H - 6, 9, 6)):  # other tile shapes, other tile corners
+            ctx.reset()
+            ctx.ppb_pass(seed=8, pass_index=0, crop=crop)
+            x0, y0, cw, ch = crop
+            np.testing.assert_array_equal(ctx.image_sum()[y0:y0 + ch, x0:x0 + cw], got[y0:y0 + ch, x0:x0 + cw])
+    want, _ = orc.ppb_pass(g, cloud, cam, prm, 300, 1 << 17, radius, 0.8, W, H, seed=8, pass_index=0)
+    np.testing.assert_array_equal(got, want)
+    assert (want > 0.0).any()
