@@ -34,6 +34,7 @@ cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, ui
 // ---------------------------------------------------------------------------
 // emission
 // ---------------------------------------------------------------------------
+constexpr uint32_t kEmitWarps = 20;  // warps of the emission an SM holds
 struct PpbEmitView {
   float* slots;         // [P * K * kSlotFloats]
   uint32_t* nbeams;     // [P]
@@ -41,7 +42,7 @@ struct PpbEmitView {
   uint32_t* slot_off;   // [P * K] exclusive prefix inside the photon
   uint32_t* photon_segs;// [P]
   float* reach;         // [P * K] the farthest of each beam's transmittance distances
-  uint32_t photons, K;
+  uint32_t photons, K, lanes;  // lanes: photons a warp
   float radius;
   uint32_t seed, pass;
 };
@@ -71,10 +72,17 @@ __device__ __forceinline__ float box_entry(const SceneView& s, f3 d, Rng& rng, f
   return at;
 }
 
-__global__ void __launch_bounds__(128) ppb_emit_kernel(GridView g, SceneView s, PpbEmitView v, Counters cnt) {
-  uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+// One lane a photon, v.lanes photons a warp.  The flights of all of a
+// photon's beams (16 transmittance distances and the interaction each) follow
+// one another in one loop over tentative collisions, so a lane whose flight
+// ends early goes on with its next one.
+__device__ __forceinline__ void emit_photons(const GridView& g, const SceneView& s, const PpbEmitView& v,
+                                             const Counters& cnt) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t p = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * v.lanes + lane;
+  const bool mine = lane < v.lanes && p < v.photons;
   uint32_t lookups = 0, cells = 0, events = 0, beams = 0;
-  if (p < v.photons) {
+  if (mine) {
     Rng rng = rng_pcg(v.seed ^ kEmitSalt, p, v.pass);
     f3 d, power;
     const float inv = 1.0f / ((float)v.photons * 0.5f);
@@ -98,41 +106,64 @@ __global__ void __launch_bounds__(128) ppb_emit_kernel(GridView g, SceneView s, 
       power = s.sky * f;
     }
     uint32_t seg_total = 0;
-    while (beams < v.K) {
-      float tmin, tmax;
-      if (!slab(o, d, s.b0, s.b1, tmin, tmax) || !finite_pos(tmax)) break;
-      // deposit a beam from o to the box exit (depositPhotonBeam, PPB_PT.comp:334-393)
-      float* sl = v.slots + ((size_t)p * v.K + beams) * kSlotFloats;
-      sl[0] = o.x; sl[1] = o.y; sl[2] = o.z;
-      sl[3] = d.x; sl[4] = d.y; sl[5] = d.z;
-      sl[6] = tmax;
-      sl[7] = power.x; sl[8] = power.y; sl[9] = power.z;
-      float reach = 0.0f;
-      for (int i = 0; i < kBeamDists; ++i) {
-        float t;
-        const float e = free_flight(g, s, o, d, rng, t, lookups, cells) ? t : kEscaped;
-        sl[10 + i] = e;
-        reach = fmaxf(reach, e);
+    int flight = 0;  // of the beam: 16 distances, then the interaction
+    bool beam = true, fresh = true;  // a beam begins; a flight begins
+    float reach = 0.0f;
+    float* sl = nullptr;
+    Track tr;
+    while (true) {
+      if (beam) {
+        float tmin, tmax;
+        if (beams >= v.K || !slab(o, d, s.b0, s.b1, tmin, tmax) || !finite_pos(tmax)) break;
+        // deposit a beam from o to the box exit (depositPhotonBeam, PPB_PT.comp:334-393)
+        const size_t slot = (size_t)p * v.K + beams;
+        sl = v.slots + slot * kSlotFloats;
+        sl[0] = o.x; sl[1] = o.y; sl[2] = o.z;
+        sl[3] = d.x; sl[4] = d.y; sl[5] = d.z;
+        sl[6] = tmax;
+        sl[7] = power.x; sl[8] = power.y; sl[9] = power.z;
+        const uint32_t ns = segments_of(tmax, v.radius);
+        v.slot_segs[slot] = ns;
+        v.slot_off[slot] = seg_total;
+        seg_total += ns;
+        ++beams;
+        reach = 0.0f;
+        flight = 0;
+        beam = false;
+        fresh = true;
       }
-      v.reach[(size_t)p * v.K + beams] = reach;
-      uint32_t ns = segments_of(tmax, v.radius);
-      v.slot_segs[(size_t)p * v.K + beams] = ns;
-      v.slot_off[(size_t)p * v.K + beams] = seg_total;
-      seg_total += ns;
-      ++beams;
+      if (fresh) track_init(tr, g, s, g.majorants, o, d, cells);
+      fresh = false;
+      float tau = -vlog(rng_next(rng));
+      bool ended = true, hit = false;
+      if (track_walk(tr, g.majorants, s.k_sigma, tau, cells, 0xFFFFFFFFu) == kCandidate) {
+        const float rho = density_at(g, s, along(o, d, tr.t));
+        ++lookups;
+        if (rng_next(rng) * tr.m < rho) hit = true;
+        else ended = lookups + cells > kPathWorkCap;  // runaway guard (non-finite input)
+      }
+      if (!ended) continue;
+      fresh = true;
+      if (flight < kBeamDists) {
+        const float e = hit ? tr.t : kEscaped;
+        sl[10 + flight] = e;
+        reach = fmaxf(reach, e);
+        if (++flight == kBeamDists) v.reach[(size_t)p * v.K + beams - 1u] = reach;
+        continue;
+      }
       // next interaction (interactWithMedium, PPB_PT.comp:453-501)
-      float t;
-      if (!free_flight(g, s, o, d, rng, t, lookups, cells)) break;
-      o = along(o, d, t);
+      if (!hit) break;
+      o = along(o, d, tr.t);
       ++events;
       power = power * s.albedo;
       if (s.max_events && events >= s.max_events) break;
       d = hg_sample(s.ph, d, rng, true);
+      beam = true;
     }
     v.nbeams[p] = beams;
     v.photon_segs[p] = seg_total;
   }
-  flush_counters(cnt, p < v.photons ? 1ull : 0ull, lookups, events, cells);
+  flush_counters(cnt, mine ? 1ull : 0ull, lookups, events, cells);
 }
 
 // One thread per (photon, beam): split into equal segments of about the
@@ -494,9 +525,9 @@ __device__ __forceinline__ void sort16(float (&v)[kBeamDists]) {
 // order.  One thread a pixel; its flights follow one another in one loop
 // over tentative collisions, so lanes whose flights end early go on with
 // their next one instead of waiting for the warp's longest.
-__global__ void __launch_bounds__(128) ppb_camera_kernel(GridView g, SceneView s, CamView cam, PassView pv,
-                                                         PpbGatherView v, Counters cnt) {
-  const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void camera_flights(const GridView& g, const SceneView& s, const CamView& cam,
+                                               const PassView& pv, const PpbGatherView& v, const Counters& cnt,
+                                               uint32_t id) {
   uint32_t lookups = 0, cells = 0;
   if (id < pv.cw * pv.ch) {
     const uint32_t cy = id / pv.cw, cx = id - cy * pv.cw;
@@ -539,6 +570,26 @@ __global__ void __launch_bounds__(128) ppb_camera_kernel(GridView g, SceneView s
     }
   }
   flush_counters(cnt, 0ull, lookups, 0, cells);
+}
+
+// The two need nothing of each other: the camera's CTAs follow the emission's
+// in one launch and fill the SMs as its longest photons end.  What bounds the
+// emission is its longest photon, some thousand flights one after the other:
+// the fewer photons share its warp, the shorter its turns, so a warp takes no
+// more of them than put every warp on the SMs at once (20 an SM).  A whole
+// pass, with one launch after the other and 32 photons a warp, and now:
+// 1280x720, 60,741 photons 23.98 -> 23.54 ms; 640x360, 20,000 photons 5.62 ->
+// 5.20; 160x90, 5,000 photons 2.35 -> 1.49 (12 warps an SM 1.58, 26 the first
+// 23.93).  Photons from a cursor, 1 to 3 CTAs an SM: 25.6 to 23.9 ms, 2.72 the
+// small one.
+__global__ void __launch_bounds__(128) ppb_trace_kernel(const __grid_constant__ GridView g,
+                                                        const __grid_constant__ SceneView s,
+                                                        const __grid_constant__ PpbEmitView ev, uint32_t emit_blocks,
+                                                        const __grid_constant__ CamView cam,
+                                                        const __grid_constant__ PassView pv,
+                                                        const __grid_constant__ PpbGatherView v, Counters cnt) {
+  if (blockIdx.x < emit_blocks) emit_photons(g, s, ev, cnt);
+  else camera_flights(g, s, cam, pv, v, cnt, (blockIdx.x - emit_blocks) * blockDim.x + threadIdx.x);
 }
 
 // A pixel tile's view of the scene, for finding the tile's pixels whose rays
@@ -1158,9 +1209,24 @@ vcr_status ppb_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
   st->radius = ppb_radius_at(st->prm.radius, st->prm.alpha, pass->pass_index);
   Counters cnt{ctx->d_counters};
   VCR_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0, 5 * sizeof(unsigned long long), st_));
-  PpbEmitView ev{st->slots, st->nbeams, st->slot_segs, st->slot_off, st->photon_segs, st->reach, P, K, st->radius,
+  PpbEmitView ev{st->slots, st->nbeams, st->slot_segs, st->slot_off, st->photon_segs, st->reach, P, K, 32u, st->radius,
                  pass->seed, pass->pass_index};
-  ppb_emit_kernel<<<(P + 127) / 128, 128, 0, st_>>>(g, s, ev, cnt);
+  const size_t pixels = (size_t)pv.cw * pv.ch;
+  if (st->cam_pixels < pixels) {  // kept for the next pass; frames may grow after the set-up
+    cudaFree(st->cam_dist);
+    st->cam_dist = nullptr;
+    st->cam_pixels = 0;
+    VCR_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&st->cam_dist), pixels * kBeamDists * sizeof(float)));
+    st->cam_pixels = pixels;
+  }
+  PpbGatherView gv{};
+  gv.cam_dist = st->cam_dist;
+  gv.seed = pass->seed;
+  gv.pass = pass->pass_index;
+  while (ev.lanes > 1u && P <= (ev.lanes / 2u) * kEmitWarps * (uint32_t)ctx->sm_count) ev.lanes /= 2u;
+  const uint32_t emit_blocks = (P + 4u * ev.lanes - 1u) / (4u * ev.lanes);
+  ppb_trace_kernel<<<emit_blocks + (unsigned)((pixels + 127) / 128), 128, 0, st_>>>(g, s, ev, emit_blocks,
+                                                                                   cam_view(ctx->cam), pv, gv, cnt);
   VCR_CUDA(ctx, cudaGetLastError());
   VCR_CUDA(ctx, exclusive_scan_u32(st->photon_segs, st->photon_off, P, st->scan_sums, st->total, st_));
   uint32_t total = 0;
@@ -1181,7 +1247,6 @@ vcr_status ppb_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
                         st->node_hi, st_, nullptr);
   if (vs) return vs;
   // the gather's leaves and clusters
-  PpbGatherView gv{};
   gv.cl = cluster_layout(n);
   gv.leaf = GatherLeaves{st->leaf_a, st->leaf_b, st->live_lo, st->live_hi, st->leaf_beam};
   gv.n_live = st->total;  // n's copy is on the host by now
@@ -1218,25 +1283,12 @@ vcr_status ppb_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
       VCR_CUDA(ctx, cudaGetLastError());
     }
   }
-  const size_t pixels = (size_t)pv.cw * pv.ch;
-  if (st->cam_pixels < pixels) {  // kept for the next pass; frames may grow after the set-up
-    cudaFree(st->cam_dist);
-    st->cam_dist = nullptr;
-    st->cam_pixels = 0;
-    VCR_CUDA(ctx, cudaMalloc(reinterpret_cast<void**>(&st->cam_dist), pixels * kBeamDists * sizeof(float)));
-    st->cam_pixels = pixels;
-  }
   gv.slots = st->slots;
   gv.radius = st->radius;
   gv.cluster_lo = st->cluster_lo;
   gv.cluster_hi = st->cluster_hi;
-  gv.cam_dist = st->cam_dist;
-  gv.seed = pass->seed;
-  gv.pass = pass->pass_index;
   vcr_status ps = probe_begin(ctx, st->gather, st_);
   if (ps) return ps;
-  ppb_camera_kernel<<<(unsigned)((pixels + 127) / 128), 128, 0, st_>>>(g, s, cam_view(ctx->cam), pv, gv, cnt);
-  VCR_CUDA(ctx, cudaGetLastError());
   vs = gather_launch(ctx, g, s, cam_view(ctx->cam), pv, gv, cnt, st->gather.d_count, st_);
   if (vs) return vs;
   ps = probe_end(ctx, st->gather, st_);

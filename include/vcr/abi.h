@@ -591,7 +591,8 @@ VCR_API vcr_status vcr_ppb_info(vcr_ctx* ctx, vcr_ppb_info_t* out);
  * of which a point may come within the radius of the pixel's ray, without
  * those that contribute exactly 0: past the beam's or the camera ray's
  * farthest transmittance sample, or in cells without density) and its device
- * time.  Waits for the gather to finish.  No reference counterpart
+ * time (the camera rays' samples are drawn with the beams, before it).  Waits
+ * for the gather to finish.  No reference counterpart
  * (measurement). */
 VCR_API vcr_status vcr_ppb_gather_stats(vcr_ctx* ctx, uint64_t* segments_evaluated, float* ms);
 /* Synchronous copy of one of the last pass's beam buffers. */

@@ -94,3 +94,27 @@ def test_segment_ranges_match_the_oracle(cuda, sun, radius):
     want, _ = orc.ppb_pass(g, cloud, cam, prm, 300, 1 << 17, radius, 0.8, W, H, seed=8, pass_index=0)
     np.testing.assert_array_equal(got, want)
     assert (want > 0.0).any()
+
+
+# photons a warp: 1 up to 20 warps an SM of 152, then 2 .. 32; a ragged last warp
+@pytest.mark.parametrize("photons", [3040, 3041, 6083, 48643])
+def test_emission_matches_the_oracle_at_every_share_of_a_warp(cuda, photons):
+    W, H, cap = 24, 17, 1 << 14
+    ctx, g, cloud, cam, prm = _context(W, H)
+    prm.max_events = 3
+    with ctx:
+        ctx.set_params(prm)
+        ctx.ppb_setup(photons, cap, 0.5, 0.8)
+        ctx.ppb_pass(seed=6, pass_index=0, crop=(W // 2, H // 2, 2, 2))
+        info = ctx.ppb_info()
+        nbeams = ctx.ppb_read("nbeams", photons)
+        slots = ctx.ppb_read("slots", photons)
+    _, ob = orc.ppb_pass(g, cloud, cam, prm, photons, cap, 0.5, 0.8, W, H, seed=6, pass_index=0,
+                         crop=(W // 2, H // 2, 2, 2))
+    assert info["segments"] == ob["info"]["segments"] and info["dropped"] == ob["info"]["dropped"]
+    np.testing.assert_array_equal(nbeams, ob["nbeams"])
+    k = slots.size // (photons * 28)
+    mine, want = slots.reshape(photons, k, 28), ob["slots"].reshape(photons, -1, 28)
+    for b in range(k):
+        has = nbeams > b
+        np.testing.assert_array_equal(mine[has, b], want[has, b])
