@@ -215,11 +215,9 @@ __device__ __forceinline__ int lbvh_delta(const uint32_t* __restrict__ keys, int
   return __clz(a ^ b);
 }
 
-__global__ void lbvh_build_kernel(const uint32_t* __restrict__ keys, int n, uint32_t* __restrict__ left,
-                                  uint32_t* __restrict__ right, uint32_t* __restrict__ parent_int,
-                                  uint32_t* __restrict__ parent_leaf) {
-  int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (i >= n - 1) return;
+// Children and leaf range [first, last] of internal node i.
+__device__ __forceinline__ void lbvh_node(const uint32_t* __restrict__ keys, int n, int i, uint32_t& left,
+                                          uint32_t& right, int& first, int& last) {
   int d = lbvh_delta(keys, n, i, i + 1) - lbvh_delta(keys, n, i, i - 1) > 0 ? 1 : -1;
   int dmin = lbvh_delta(keys, n, i, i - d);
   int lmax = 2;
@@ -236,15 +234,21 @@ __global__ void lbvh_build_kernel(const uint32_t* __restrict__ keys, int n, uint
     if (t == 1) break;
   }
   int gamma = i + s * d + (d < 0 ? -1 : 0);
-  uint32_t lc = (min(i, j) == gamma) ? ((uint32_t)gamma | kLeafBit) : (uint32_t)gamma;
-  uint32_t rc = (max(i, j) == gamma + 1) ? ((uint32_t)(gamma + 1) | kLeafBit) : (uint32_t)(gamma + 1);
-  left[i] = lc;
-  right[i] = rc;
-  if (lc & kLeafBit) parent_leaf[lc & ~kLeafBit] = (uint32_t)i;
-  else parent_int[lc] = (uint32_t)i;
-  if (rc & kLeafBit) parent_leaf[rc & ~kLeafBit] = (uint32_t)i;
-  else parent_int[rc] = (uint32_t)i;
-  if (i == 0) parent_int[0] = 0xFFFFFFFFu;
+  first = min(i, j);
+  last = max(i, j);
+  left = first == gamma ? (uint32_t)gamma | kLeafBit : (uint32_t)gamma;
+  right = last == gamma + 1 ? (uint32_t)(gamma + 1) | kLeafBit : (uint32_t)(gamma + 1);
+}
+
+__global__ void lbvh_build_kernel(const uint32_t* __restrict__ keys, int n, uint32_t* __restrict__ left,
+                                  uint32_t* __restrict__ right) {
+  int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (i >= n - 1) return;
+  uint32_t l, r;
+  int first, last;
+  lbvh_node(keys, n, i, l, r, first, last);
+  left[i] = l;
+  right[i] = r;
 }
 
 // Capped-cylinder AABB of a segment (calculateBeamBounds,
@@ -392,54 +396,132 @@ __global__ void __launch_bounds__(256) ppb_cluster_kernel(const float4* __restri
   }
 }
 
-// Arrival counter of the refit: an atomic add with acquire-release
-// semantics at GPU scope, so the box a thread stored before its arrival is
-// visible to the sibling that arrives second, without separate fences.
-__device__ __forceinline__ uint32_t arrive_acq_rel(uint32_t* p) {
-  uint32_t old;
-  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
-  return old;
+// A node's box is the union of the leaf boxes of its range, whatever the tree
+// between them looks like, so the nodes need not wait for one another: short
+// ranges are read leaf by leaf, longer ones are taken by the whole warp from
+// boxes over 32, 32^2 and 32^3 leaves (clusters).  Minima and maxima: the
+// values of a walk from the leaves up.  9.6 M leaves, topology and boxes: 774 us,
+// bound by the loads of the searches and ranges (1,254 us with the second
+// child to arrive at a node, by an atomic counter, taking its box up).
+constexpr int kLbvhLevels = 4;   // leaves, and three levels of clusters
+constexpr int kLbvhShort = 32;   // leaves a lane reads itself (8 / 16 / 32 / 64: 700 / 619 / 606 / 630 us)
+struct LbvhBoxes {
+  const float4* lo[kLbvhLevels];
+  const float4* hi[kLbvhLevels];
+};
+
+__device__ __forceinline__ void box_add(float4& lo, float4& hi, const float4 l, const float4 h) {
+  lo.x = fminf(lo.x, l.x);
+  lo.y = fminf(lo.y, l.y);
+  lo.z = fminf(lo.z, l.z);
+  hi.x = fmaxf(hi.x, h.x);
+  hi.y = fmaxf(hi.y, h.y);
+  hi.z = fmaxf(hi.z, h.z);
 }
 
-// Leaf boxes, then a bottom-up walk: the second child to arrive at a node
-// (atomic counter) computes its box from both children and moves up; it
-// holds its own child's box and loads only the sibling's.
-__global__ void lbvh_refit_kernel(const float4* __restrict__ seg_a, const float4* __restrict__ seg_b,
-                                  const uint32_t* __restrict__ order, int n, const uint32_t* __restrict__ left,
-                                  const uint32_t* __restrict__ right, const uint32_t* __restrict__ parent_int,
-                                  const uint32_t* __restrict__ parent_leaf, uint32_t* __restrict__ flags,
-                                  float4* __restrict__ leaf_lo, float4* __restrict__ leaf_hi,
-                                  float4* __restrict__ node_lo, float4* __restrict__ node_hi,
-                                  float4* __restrict__ node_pk) {
-  int g = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (g >= n) return;
-  uint32_t sid = order[g];
+// Leaf boxes, and the clusters of 32 and of 1,024 of them.
+__global__ void __launch_bounds__(1024) lbvh_leaf_kernel(const float4* __restrict__ seg_a,
+                                                         const float4* __restrict__ seg_b,
+                                                         const uint32_t* __restrict__ order, int n,
+                                                         float4* __restrict__ leaf_lo, float4* __restrict__ leaf_hi,
+                                                         float4* __restrict__ lo1, float4* __restrict__ hi1,
+                                                         float4* __restrict__ lo2, float4* __restrict__ hi2) {
+  __shared__ float4 s_lo[32], s_hi[32];
+  const int g = (int)(blockIdx.x * blockDim.x + threadIdx.x), lane = (int)(threadIdx.x & 31u);
+  const int warp = (int)(threadIdx.x >> 5);
+  const uint32_t sid = order[min(g, n - 1)];  // past the end: the last leaf again
   float4 lo, hi;
   segment_box(seg_a[sid], seg_b[sid], lo, hi);
-  leaf_lo[g] = lo;
-  leaf_hi[g] = hi;
-  if (n == 1) return;
-  uint32_t me = (uint32_t)g | kLeafBit;  // the child this thread climbs from, and its box (lo, hi)
-  uint32_t node = parent_leaf[g];
-  for (int guard = 0; node != 0xFFFFFFFFu && guard < 64; ++guard) {
-    if (arrive_acq_rel(flags + node) == 0u) return;  // first arrival: the sibling finishes this node
-    const uint32_t l = left[node], r = right[node];
-    const bool mine_left = l == me;
-    const uint32_t sib = mine_left ? r : l;
-    const float4 slo = (sib & kLeafBit) ? __ldcg(leaf_lo + (sib & ~kLeafBit)) : __ldcg(node_lo + sib);
-    const float4 shi = (sib & kLeafBit) ? __ldcg(leaf_hi + (sib & ~kLeafBit)) : __ldcg(node_hi + sib);
-    const float4 al = mine_left ? lo : slo, ah = mine_left ? hi : shi;  // left child's box
-    const float4 bl = mine_left ? slo : lo, bh = mine_left ? shi : hi;  // right child's box
-    lo = make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), 0.f);
-    hi = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), 0.f);
-    node_lo[node] = lo;
-    node_hi[node] = hi;
-    if (node_pk) {  // box and children together: one 32-byte sector per node for the gathers
-      node_pk[2 * (size_t)node] = make_float4(lo.x, lo.y, lo.z, __uint_as_float(l));
-      node_pk[2 * (size_t)node + 1] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(r));
+  if (g < n) {
+    leaf_lo[g] = lo;
+    leaf_hi[g] = hi;
+  }
+  if (!lo1) return;
+  warp_box(lo, hi);
+  if (lane == 0) {
+    if (g < n) {
+      lo1[g >> 5] = lo;
+      hi1[g >> 5] = hi;
     }
-    me = node;
-    node = parent_int[node];
+    s_lo[warp] = lo;
+    s_hi[warp] = hi;
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  lo = s_lo[lane];
+  hi = s_hi[lane];
+  warp_box(lo, hi);
+  if (lane == 0) {
+    lo2[blockIdx.x] = lo;
+    hi2[blockIdx.x] = hi;
+  }
+}
+
+// Clusters of 32 boxes, a warp each.
+__global__ void lbvh_cluster_kernel(const float4* __restrict__ lo_in, const float4* __restrict__ hi_in, int n,
+                                    float4* __restrict__ lo_out, float4* __restrict__ hi_out) {
+  const int lane = (int)(threadIdx.x & 31u), c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (c * 32 >= n) return;  // warp-uniform
+  const int i = min(c * 32 + lane, n - 1);
+  float4 lo = lo_in[i], hi = hi_in[i];
+  warp_box(lo, hi);
+  if (lane == 0) {
+    lo_out[c] = lo;
+    hi_out[c] = hi;
+  }
+}
+
+__global__ void __launch_bounds__(256) lbvh_node_kernel(const uint32_t* __restrict__ keys, int n, LbvhBoxes b,
+                                                        uint32_t* __restrict__ left, uint32_t* __restrict__ right,
+                                                        float4* __restrict__ node_lo, float4* __restrict__ node_hi,
+                                                        float4* __restrict__ node_pk) {
+  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x), lane = (int)(threadIdx.x & 31u);
+  const bool mine = i < n - 1;
+  uint32_t l = 0, r = 0;
+  int first = 0, last = 0;
+  float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+  if (mine) {
+    lbvh_node(keys, n, i, l, r, first, last);
+    if (last - first < kLbvhShort) {
+      lo = b.lo[0][first];
+      hi = b.hi[0][first];
+      for (int k = first + 1; k <= last; ++k) box_add(lo, hi, b.lo[0][k], b.hi[0][k]);
+    }
+  }
+  for (uint32_t todo = __ballot_sync(0xffffffffu, mine && last - first >= kLbvhShort); todo; todo &= todo - 1u) {
+    const int src = __ffs(todo) - 1;
+    int p = __shfl_sync(0xffffffffu, first, src), e = __shfl_sync(0xffffffffu, last, src) + 1;
+    // the range's ends at a level that a cluster of the next does not cover,
+    // then the clusters between them
+    float4 wl = b.lo[0][p], wh = b.hi[0][p];
+#pragma unroll
+    for (int level = 0; level < kLbvhLevels; ++level) {
+      const float4* bl = b.lo[level];
+      const float4* bh = b.hi[level];
+      if (level + 1 == kLbvhLevels || e - p <= 64) {
+        for (int k = p + lane; k < e; k += 32) box_add(wl, wh, bl[k], bh[k]);
+        break;
+      }
+      const int up = (p + 31) & ~31, down = e & ~31;  // up <= down: the range is longer than 64
+      if (p + lane < up) box_add(wl, wh, bl[p + lane], bh[p + lane]);
+      if (down + lane < e) box_add(wl, wh, bl[down + lane], bh[down + lane]);
+      p = up >> 5;
+      e = down >> 5;
+    }
+    warp_box(wl, wh);
+    if (lane == src) {
+      lo = wl;
+      hi = wh;
+    }
+  }
+  if (!mine) return;
+  left[i] = l;
+  right[i] = r;
+  node_lo[i] = make_float4(lo.x, lo.y, lo.z, 0.f);
+  node_hi[i] = make_float4(hi.x, hi.y, hi.z, 0.f);
+  if (node_pk) {  // box and children together: one 32-byte sector per node for the gathers
+    node_pk[2 * (size_t)i] = make_float4(lo.x, lo.y, lo.z, __uint_as_float(l));
+    node_pk[2 * (size_t)i + 1] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(r));
   }
 }
 
@@ -1098,7 +1180,7 @@ static void ppb_release(PpbState* st) {
                   st->photon_off, st->scan_sums,   st->total,       st->seg_a,      st->seg_b,
                   st->leaf_a,     st->leaf_b,      st->leaf_beam,   st->cluster_lo, st->seg_beam,
                   st->codes,      st->idx,         st->codes_sorted, st->idx_sorted, st->left,
-                  st->right,      st->parent_int,  st->parent_leaf, st->flags,      st->leaf_lo,
+                  st->right,      st->tree_clusters, st->live_counts, st->leaf_lo,
                   st->leaf_hi,    st->node_lo,     st->node_hi,     st->cluster_hi, st->cam_dist,
                   st->live_lo,    st->live_hi,     st->live_mask,   st->live_off,   st->reach};
   for (void* p : ptrs) cudaFree(p);
@@ -1118,6 +1200,14 @@ float ppb_radius_at(float r0, float alpha, uint32_t pass) {
   double r = r0;
   for (uint32_t i = 1; i <= pass; ++i) r *= ((double)i + (double)alpha) / ((double)i + 1.0);
   return (float)r;
+}
+
+// Cluster boxes of a tree of n leaves.
+static int lbvh_count(int n, int level) { return (int)(((int64_t)n + (1ll << (5 * level)) - 1) >> (5 * level)); }
+size_t lbvh_cluster_bytes(size_t n) {
+  size_t boxes = 0;
+  for (int l = 1; l < kLbvhLevels; ++l) boxes += (n + ((size_t)1 << (5 * l)) - 1) >> (5 * l);
+  return boxes * 2 * sizeof(float4);
 }
 
 vcr_status ppb_setup(vcr_ctx* ctx, const vcr_ppb_params* p) {
@@ -1160,9 +1250,8 @@ vcr_status ppb_setup(vcr_ctx* ctx, const vcr_ppb_params* p) {
   VCR_ALLOC(st->idx_sorted, C * 4);
   VCR_ALLOC(st->left, C * 4);
   VCR_ALLOC(st->right, C * 4);
-  VCR_ALLOC(st->parent_int, C * 4);
-  VCR_ALLOC(st->parent_leaf, C * 4);
-  VCR_ALLOC(st->flags, C * 4);
+  VCR_ALLOC(st->tree_clusters, lbvh_cluster_bytes(C));
+  VCR_ALLOC(st->live_counts, (C + 31) / 32 * 4);
   VCR_ALLOC(st->leaf_lo, C * sizeof(float4));
   VCR_ALLOC(st->leaf_hi, C * sizeof(float4));
   VCR_ALLOC(st->node_lo, C * sizeof(float4));
@@ -1171,24 +1260,39 @@ vcr_status ppb_setup(vcr_ctx* ctx, const vcr_ppb_params* p) {
   return ensure_scratch(ctx, sort_scratch_bytes(p->capacity));
 }
 
-vcr_status lbvh_build(vcr_ctx* ctx, const uint32_t* codes, int n, uint32_t* left, uint32_t* right,
-                      uint32_t* parent_int, uint32_t* parent_leaf, cudaStream_t st) {
+vcr_status lbvh_build(vcr_ctx* ctx, const uint32_t* codes, int n, uint32_t* left, uint32_t* right, cudaStream_t st) {
   if (n <= 1) return VCR_OK;
-  lbvh_build_kernel<<<(n - 1 + 255) / 256, 256, 0, st>>>(codes, n, left, right, parent_int, parent_leaf);
+  lbvh_build_kernel<<<(n - 1 + 255) / 256, 256, 0, st>>>(codes, n, left, right);
   VCR_CUDA(ctx, cudaGetLastError());
   return VCR_OK;
 }
 
 vcr_status lbvh_build_refit(vcr_ctx* ctx, const uint32_t* codes, const uint32_t* order, const float4* seg_a,
-                            const float4* seg_b, int n, uint32_t* left, uint32_t* right, uint32_t* parent_int,
-                            uint32_t* parent_leaf, uint32_t* flags, float4* leaf_lo, float4* leaf_hi,
-                            float4* node_lo, float4* node_hi, cudaStream_t st, float4* node_pk) {
+                            const float4* seg_b, int n, uint32_t* left, uint32_t* right, float4* clusters,
+                            float4* leaf_lo, float4* leaf_hi, float4* node_lo, float4* node_hi, cudaStream_t st,
+                            float4* node_pk) {
   if (n <= 0) return VCR_OK;
-  vcr_status vs = lbvh_build(ctx, codes, n, left, right, parent_int, parent_leaf, st);
-  if (vs) return vs;
-  if (n > 1) VCR_CUDA(ctx, cudaMemsetAsync(flags, 0, (size_t)(n - 1) * 4, st));
-  lbvh_refit_kernel<<<(n + 255) / 256, 256, 0, st>>>(seg_a, seg_b, order, n, left, right, parent_int, parent_leaf,
-                                                     flags, leaf_lo, leaf_hi, node_lo, node_hi, node_pk);
+  LbvhBoxes b{};
+  float4 *lo[kLbvhLevels] = {leaf_lo}, *hi[kLbvhLevels] = {leaf_hi};
+  const bool clustered = n > 64;  // shorter ranges are read leaf by leaf
+  for (int l = 1; l < kLbvhLevels && clustered; ++l) {
+    lo[l] = clusters;
+    hi[l] = clusters + lbvh_count(n, l);
+    clusters += 2 * (size_t)lbvh_count(n, l);
+  }
+  lbvh_leaf_kernel<<<lbvh_count(n, 2), 1024, 0, st>>>(seg_a, seg_b, order, n, leaf_lo, leaf_hi, lo[1], hi[1], lo[2], hi[2]);
+  VCR_CUDA(ctx, cudaGetLastError());
+  if (clustered) {
+    const int boxes = lbvh_count(n, 2);
+    lbvh_cluster_kernel<<<(lbvh_count(n, 3) + 7) / 8, 256, 0, st>>>(lo[2], hi[2], boxes, lo[3], hi[3]);
+    VCR_CUDA(ctx, cudaGetLastError());
+  }
+  if (n == 1) return VCR_OK;
+  for (int l = 0; l < kLbvhLevels; ++l) {
+    b.lo[l] = lo[l];
+    b.hi[l] = hi[l];
+  }
+  lbvh_node_kernel<<<(n - 1 + 255) / 256, 256, 0, st>>>(codes, n, b, left, right, node_lo, node_hi, node_pk);
   VCR_CUDA(ctx, cudaGetLastError());
   return VCR_OK;
 }
@@ -1243,8 +1347,7 @@ vcr_status ppb_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
   VCR_CUDA(ctx, sort_pairs_enqueue(ctx->sm_count, ctx->d_error, ctx->d_scratch, st->codes, st->idx, st->codes_sorted,
                                    st->idx_sorted, n, 0, 30, st_));
   vs = lbvh_build_refit(ctx, st->codes_sorted, st->idx_sorted, st->seg_a, st->seg_b, (int)n, st->left, st->right,
-                        st->parent_int, st->parent_leaf, st->flags, st->leaf_lo, st->leaf_hi, st->node_lo,
-                        st->node_hi, st_, nullptr);
+                        st->tree_clusters, st->leaf_lo, st->leaf_hi, st->node_lo, st->node_hi, st_, nullptr);
   if (vs) return vs;
   // the gather's leaves and clusters
   gv.cl = cluster_layout(n);
@@ -1267,9 +1370,9 @@ vcr_status ppb_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
     for (int a = 0; a < 3; ++a) lv.mnb[a] = ctx->mnb[level][a];
     lv.icell = mk(1.0f / cell.x, 1.0f / cell.y, 1.0f / cell.z);
     const uint32_t c = (n + 31u) / 32u;
-    ppb_live_kernel<<<(c + 7u) / 8u, 256, 0, st_>>>(lv, n, st->live_mask, st->flags);
+    ppb_live_kernel<<<(c + 7u) / 8u, 256, 0, st_>>>(lv, n, st->live_mask, st->live_counts);
     VCR_CUDA(ctx, cudaGetLastError());
-    VCR_CUDA(ctx, exclusive_scan_u32(st->flags, st->live_off, c, st->scan_sums, st->total, st_));
+    VCR_CUDA(ctx, exclusive_scan_u32(st->live_counts, st->live_off, c, st->scan_sums, st->total, st_));
     ppb_compact_kernel<<<(c + 7u) / 8u, 256, 0, st_>>>(st->idx_sorted, st->seg_a, st->seg_b, st->seg_beam,
                                                        st->leaf_lo, st->leaf_hi, n, st->live_mask, st->live_off,
                                                        gv.leaf);
@@ -1385,17 +1488,14 @@ extern "C" VCR_API vcr_status vcr_lbvh_build(vcr_ctx* ctx, const uint32_t* d_sor
       (n > 1 && (!d_left || !d_right || !d_node_lo || !d_node_hi)))
     return fail(ctx, VCR_ERR_INVALID, "null LBVH buffer");
   VCR_CUDA(ctx, cudaSetDevice(ctx->device));
-  size_t need = (size_t)3 * n * 4;  // parent_int, parent_leaf, flags
-  vcr_status vs = ensure_scratch(ctx, need);
+  vcr_status vs = ensure_scratch(ctx, lbvh_cluster_bytes(n));
   if (vs) return vs;
-  uint32_t* pi = reinterpret_cast<uint32_t*>(ctx->d_scratch);
-  uint32_t* pl = pi + n;
-  uint32_t* fl = pl + n;
   cudaStream_t st = (cudaStream_t)stream;
   vs = lbvh_build_refit(ctx, d_sorted_codes, d_order, reinterpret_cast<const float4*>(d_seg_a),
-                        reinterpret_cast<const float4*>(d_seg_b), (int)n, d_left, d_right, pi, pl, fl,
-                        reinterpret_cast<float4*>(d_leaf_lo), reinterpret_cast<float4*>(d_leaf_hi),
-                        reinterpret_cast<float4*>(d_node_lo), reinterpret_cast<float4*>(d_node_hi), st, nullptr);
+                        reinterpret_cast<const float4*>(d_seg_b), (int)n, d_left, d_right,
+                        reinterpret_cast<float4*>(ctx->d_scratch), reinterpret_cast<float4*>(d_leaf_lo),
+                        reinterpret_cast<float4*>(d_leaf_hi), reinterpret_cast<float4*>(d_node_lo),
+                        reinterpret_cast<float4*>(d_node_hi), st, nullptr);
   if (vs) return vs;
   VCR_CUDA(ctx, cudaEventRecord(ctx->work_done, st));
   return VCR_OK;

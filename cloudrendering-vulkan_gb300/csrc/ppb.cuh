@@ -33,7 +33,8 @@ struct PpbState {
   uint32_t *leaf_beam = nullptr, *live_mask = nullptr, *live_off = nullptr;  // the latter two per 32 leaves
   float* reach = nullptr;  // per beam slot: the farthest of its transmittance distances
   uint32_t *seg_beam = nullptr, *codes = nullptr, *idx = nullptr, *codes_sorted = nullptr, *idx_sorted = nullptr;
-  uint32_t *left = nullptr, *right = nullptr, *parent_int = nullptr, *parent_leaf = nullptr, *flags = nullptr;
+  uint32_t *left = nullptr, *right = nullptr, *live_counts = nullptr;
+  float4* tree_clusters = nullptr;  // boxes over 32, 32^2 and 32^3 leaves while the tree is built
   float4 *leaf_lo = nullptr, *leaf_hi = nullptr, *node_lo = nullptr, *node_hi = nullptr;
   // the gather's clusters: boxes over 32 consecutive of those, over 32 of these, ...
   float4 *cluster_lo = nullptr, *cluster_hi = nullptr;

@@ -30,12 +30,12 @@
 
 namespace vcr {
 
-vcr_status lbvh_build(vcr_ctx* ctx, const uint32_t* codes, int n, uint32_t* left, uint32_t* right,
-                      uint32_t* parent_int, uint32_t* parent_leaf, cudaStream_t st);
+vcr_status lbvh_build(vcr_ctx* ctx, const uint32_t* codes, int n, uint32_t* left, uint32_t* right, cudaStream_t st);
+size_t lbvh_cluster_bytes(size_t n);
 vcr_status lbvh_build_refit(vcr_ctx* ctx, const uint32_t* codes, const uint32_t* order, const float4* seg_a,
-                            const float4* seg_b, int n, uint32_t* left, uint32_t* right, uint32_t* parent_int,
-                            uint32_t* parent_leaf, uint32_t* flags, float4* leaf_lo, float4* leaf_hi,
-                            float4* node_lo, float4* node_hi, cudaStream_t st, float4* node_pk);
+                            const float4* seg_b, int n, uint32_t* left, uint32_t* right, float4* clusters,
+                            float4* leaf_lo, float4* leaf_hi, float4* node_lo, float4* node_hi, cudaStream_t st,
+                            float4* node_pk);
 
 cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* sums, uint32_t* d_total,
                                cudaStream_t st);
@@ -693,7 +693,7 @@ void ppm_free(vcr_ctx* ctx) {
   PpmState* st = ctx->ppm;
   if (!st) return;
   void* ptrs[] = {st->pos, st->pw, st->dir, st->uid, st->count, st->by_uid, st->uid_sorted, st->codes, st->idx,
-                  st->codes_sorted, st->order, st->left, st->right, st->parent_int, st->parent_leaf, st->flags,
+                  st->codes_sorted, st->order, st->left, st->right, st->tree_clusters,
                   st->leaf_lo, st->leaf_hi, st->node_lo, st->node_hi, st->node_pk, st->leaf_pw, st->leaf_dir,
                   st->box, st->stats, st->iota, st->points, st->point, st->point_pix,
                   st->deposits, st->first, st->scan_sums};
@@ -735,12 +735,10 @@ vcr_status ppm_setup(vcr_ctx* ctx, const vcr_ppm_params* p) {
   VCR_ALLOC(st->order, C * 4);
   VCR_ALLOC(st->left, C * 4);
   VCR_ALLOC(st->right, C * 4);
-  VCR_ALLOC(st->parent_int, C * 4);
-  VCR_ALLOC(st->parent_leaf, C * 4);
   VCR_ALLOC(st->leaf_lo, C * 16);
   VCR_ALLOC(st->box, (size_t)oct_layout(p->capacity).total * 32 + 8 * 32);  // a visit reads 8 boxes
   if (p->estimator == VCR_PPM_MARCH) {  // the march walks the tree's boxes and leaf-order photons
-    VCR_ALLOC(st->flags, C * 4);
+    VCR_ALLOC(st->tree_clusters, lbvh_cluster_bytes(C));
     VCR_ALLOC(st->leaf_hi, C * 16);
     VCR_ALLOC(st->node_lo, C * 16);
     VCR_ALLOC(st->node_hi, C * 16);
@@ -854,8 +852,7 @@ vcr_status ppm_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
   gv.pass = pass->pass_index;
   if (march) {
     vs = lbvh_build_refit(ctx, st->codes_sorted, st->order, st->pos, st->pos, (int)n, st->left, st->right,
-                          st->parent_int, st->parent_leaf, st->flags, st->leaf_lo, st->leaf_hi, st->node_lo,
-                          st->node_hi, cs, st->node_pk);
+                          st->tree_clusters, st->leaf_lo, st->leaf_hi, st->node_lo, st->node_hi, cs, st->node_pk);
     if (vs) return vs;
     if (n) {  // powers and directions in leaf order, read with the leaf's position
       ppm_leaf_order_kernel<<<ctx->sm_count * 8, 256, 0, cs>>>(st->order, st->pw, st->dir, n, st->leaf_pw,
@@ -866,7 +863,7 @@ vcr_status ppm_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
     gv.dir = st->leaf_dir;
     gv.node_pk = st->node_pk;
   } else {  // the tree's topology (readable), and the clusters the gather descends
-    vs = lbvh_build(ctx, st->codes_sorted, (int)n, st->left, st->right, st->parent_int, st->parent_leaf, cs);
+    vs = lbvh_build(ctx, st->codes_sorted, (int)n, st->left, st->right, cs);
     if (vs) return vs;
     gv.ol = oct_layout(n);
     uint32_t inputs = n;

@@ -18,7 +18,8 @@ struct PpmState {
   uint32_t *uid = nullptr, *count = nullptr, *by_uid = nullptr, *uid_sorted = nullptr, *codes = nullptr,
            *idx = nullptr, *codes_sorted = nullptr, *order = nullptr, *iota = nullptr;
   uint32_t *deposits = nullptr, *first = nullptr, *scan_sums = nullptr;  // per emitted photon: deposits, their sums
-  uint32_t *left = nullptr, *right = nullptr, *parent_int = nullptr, *parent_leaf = nullptr, *flags = nullptr;
+  uint32_t *left = nullptr, *right = nullptr;
+  float4* tree_clusters = nullptr;  // the march's tree: boxes over 32, 32^2 and 32^3 leaves while it is built
   float4 *leaf_lo = nullptr, *leaf_hi = nullptr, *node_lo = nullptr, *node_hi = nullptr;
   // the march's tree walk: internal nodes packed as (lo, left), (hi, right),
   // photon powers and directions in leaf order
