@@ -6,13 +6,13 @@
 // Tensor cores, BF16 operands, FP32 accumulation.  Queries: a
 // register-resident forward (mma.sync m16n8k16, nrc_mma.cuh) — each warp
 // runs 16-sample tiles whose activations stay in the MMA fragments, the CTA
-// shares only the BF16 weights.  Training: one 8-warp CTA per
-// SM holds the BF16 weights and, for a 128-sample tile, the six activation
-// tiles and the gradient ping-pong in padded shared memory (197 KB); the
-// forward and the backward's dY_l W_l^T run register-resident on the same
-// mma.sync fragments, and ldmatrix.trans feeds X_l^T dY_l over the tile.
-// The weight gradient stays in the warps' accumulator fragments (each warp
-// owns a 16x32 block of every hidden layer) across all the CTA's tiles; at
+// shares only the BF16 weights.  Training: one CTA per SM holds
+// the BF16 weights and, for a 128-sample tile, the activation tiles and the
+// gradient ping-pong in padded shared memory (215 KB); its warps have roles:
+// the forward and the backward's dY_l W_l^T run register-resident on the same
+// mma.sync fragments, ldmatrix.trans feeds X_l^T dY_l over the tile to warps
+// of their own, and others encode the next tile's inputs.  The weight gradient
+// stays in the warps' accumulator fragments across all the CTA's tiles; at
 // the end each CTA stores it into its own slot and one kernel sums the
 // slots in a fixed order and takes the Adam step (one atomic add per
 // weight per CTA cost as much as the tiles themselves).  Adam runs on FP32

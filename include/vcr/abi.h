@@ -235,8 +235,8 @@ VCR_API vcr_status vcr_synchronize(vcr_ctx* ctx);
  * sets the device error word, which vcr_synchronize (or, for the
  * allocation-free sort, vcr_sort_noalloc_status) reports as
  * VCR_ERR_TIMEOUT; a sort whose wait ran out has an unspecified order (it
- * stays inside its output buffers), a pass whose staging wait ran out reads
- * the majorants from global memory and renders the same image.  The limits
+ * stays inside its output buffers), a pass whose staging wait ran out
+ * copies the majorants with plain loads and renders the same image.  The limits
  * are process-wide and apply to launches queued after the call; NULL
  * restores the defaults.  Small limits exist to test the timeout path. */
 typedef struct vcr_wait_limits {
