@@ -534,8 +534,9 @@ VCR_API vcr_status vcr_ppm_free(vcr_ctx* ctx);
  * current estimate times the pass count. */
 VCR_API vcr_status vcr_ppm_pass(vcr_ctx* ctx, const vcr_pass_desc* pass, void* stream);
 VCR_API vcr_status vcr_ppm_info(vcr_ctx* ctx, vcr_ppm_info_t* out);
-/* The last pass's gather kernel: leaf photons it tested against the
- * pixels' radii and its device time (two events around the launch).
+/* The last pass's gather: photons it tested against the pixels' radii (all
+ * eight of a box that a pixel's sphere meets) and its device time, with the
+ * camera rays' (two events around the launches).
  * Waits for the gather to finish.  No reference counterpart (measurement). */
 VCR_API vcr_status vcr_ppm_gather_stats(vcr_ctx* ctx, uint64_t* photons_tested, float* ms);
 VCR_API vcr_status vcr_ppm_read(vcr_ctx* ctx, vcr_ppm_buffer which, void* host_out, size_t bytes);
