@@ -280,8 +280,9 @@ __device__ __forceinline__ bool cache_vertex(PathPool& pool, uint32_t slot, cons
 // follow.  kBatch: the camera paths are those of bt's views (pid holds the
 // view, whose sun the path uses), the view table sits in shared memory
 // after the staged majorants, and the pass index adds *bt.pass_ctr (so a
-// replayed graph renders consecutive passes).
-template <int kThreads, bool kStage, bool kBatch>
+// replayed graph renders consecutive passes).  kCache: the launch has training
+// paths, or its camera paths end in cache queries.
+template <int kThreads, bool kStage, bool kBatch, bool kCache>
 __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
     pt_wavefront_kernel(const __grid_constant__ GridView g, const __grid_constant__ SceneView s,
                         const __grid_constant__ CamView cam, const __grid_constant__ PassView pv,
@@ -319,7 +320,8 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
   const uint32_t slots = cap < 32u ? cap : (uint32_t)kPool;
   uint32_t n_free = slots, n_done = 0, n_ready = 0, h_ready = 0, n_shade = 0, h_shade = 0;
   bool exhausted = false;
-  bool serving = (threadIdx.x >> 5) * gridDim.x + blockIdx.x < train_warps;
+  const uint32_t n_train = kCache ? ts.paths : 0u;
+  bool serving = kCache && (threadIdx.x >> 5) * gridDim.x + blockIdx.x < train_warps;
   for (uint32_t i = lane; i < (uint32_t)kPool; i += 32u) pool.free_[i] = (uint8_t)i;
   if (lane < 4u) pool.totals[lane] = 0ull;
   __syncwarp();
@@ -356,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
             f3 L = mk(l, l, l);
             if (pool.T[q] != 0.0f)
               L = L + escape_radiance(s, mk(pool.dx[q], pool.dy[q], pool.dz[q])) * pool.beta[q];
-            if (pid & kTrainPath) {
+            if (kCache && (pid & kTrainPath)) {
               finish_training(ts, pix, L);
             } else {
               write_result(pv, sum, pix, L);
@@ -395,7 +397,7 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
             Rng rng{pool.rng[q], 0u};
             if (s.max_events && ev >= s.max_events) {
               end = true;
-            } else if ((pid & kTrainPath) && ts.survival > 0.0f && ev >= (uint32_t)kNrcRecordEvents &&
+            } else if (kCache && (pid & kTrainPath) && ts.survival > 0.0f && ev >= (uint32_t)kNrcRecordEvents &&
                        !roulette_survives(rng, ts.survival, beta)) {
               end = true;  // past the recorded vertices: Russian roulette
             } else if (pool.lookups[q] + pool.cells[q] > kPathWorkCap) {  // runaway guard (non-finite input)
@@ -423,8 +425,8 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
           const uint32_t take = min(min(n_free, cap), 32u);
           uint32_t base = 0;
           if (lane == 0) base = (uint32_t)atomicAdd(cnt.c + (serving ? 6 : 4), (unsigned long long)take);
-          base = __shfl_sync(0xffffffffu, base, 0) + (serving || !train_warps ? 0u : ts.paths);
-          const uint32_t end = serving ? ts.paths : total + ts.paths;
+          base = __shfl_sync(0xffffffffu, base, 0) + (serving || !kCache || !train_warps ? 0u : n_train);
+          const uint32_t end = serving ? n_train : total + n_train;
           exhausted = base + take >= end;
           uint32_t id = base + lane, pid = 0, pix = 0;
           bool hit = false;
@@ -450,7 +452,7 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
               rng = rng_pcg(pv.seed + kViewSeedStep * lo, lp * pv.spp + sp, pass);
               ps = start_path(bv.cam, s, (int)cx, (int)cy);
               if (!ps.hit) write_result(pv, sum, pix, ps.L);
-            } else if (id < ts.paths) {  // training path from a uniformly drawn pixel of the crop
+            } else if (kCache && id < n_train) {  // training path from a uniformly drawn pixel of the crop
               rng = rng_pcg(pv.seed ^ kNrcTrainSalt, id, pass);
               uint32_t pp = (uint32_t)(rng_next(rng) * (float)(pv.cw * pv.ch));
               pp = min(pp, pv.cw * pv.ch - 1u);
@@ -458,7 +460,7 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
               pix = kNrcNoSlot;
               ps = start_path(cam, s, (int)(pv.x0 + pp % pv.cw), (int)(pv.y0 + pp / pv.cw));
             } else {
-              id -= ts.paths;
+              id -= n_train;
               uint32_t pq = pass;  // a launch of several passes: item id / per_pass is the pass offset
               if (pv.passes > 1u) {
                 const uint32_t q = id / per_pass;
@@ -533,7 +535,7 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
       if (!__any_sync(0xffffffffu, mode == kFly)) {
         // nothing waits either unless it is finished paths
         if (n_done == 0u) {
-          if (!serving) break;
+          if (!kCache || !serving) break;
           serving = false;  // its training paths are done: camera paths from now on
           exhausted = total == 0u;
         }
@@ -584,7 +586,7 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
           pool.px[slot] = o.x;
           pool.py[slot] = o.y;
           pool.pz[slot] = o.z;
-          if (s.nrc_events || ts.paths) end = cache_vertex(pool, slot, s, nq, ts, o, rd);
+          if (kCache) end = cache_vertex(pool, slot, s, nq, ts, o, rd);
           T = 1.0f;
           sun_ray = true;
           rd = kBatch ? -s_views[pool.pid[slot]].sun : lsun0;
@@ -628,11 +630,11 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
 // 512^3 cloud over 16 KB of level-2 cells: 7.5 ms staged, 7.8 ms not.
 constexpr uint32_t max_staged_bytes(uint32_t threads) { return 64u * threads; }
 
-template <int kThreads, bool kStage, bool kBatch>
+template <int kThreads, bool kStage, bool kBatch, bool kCache>
 static vcr_status launch_t(vcr_ctx* ctx, const GridView& g, const SceneView& s, const CamView& cam,
                            const PassView& pv, uint32_t* stats, Counters cnt, uint32_t total, uint32_t maj_bytes,
                            const NrcTrainSink& ts, const BatchSink& bt, double* sum, cudaStream_t st) {
-  auto kern = pt_wavefront_kernel<kThreads, kStage, kBatch>;
+  auto kern = pt_wavefront_kernel<kThreads, kStage, kBatch, kCache>;
   constexpr uint32_t kWarps = kThreads / 32;
   const size_t pools = kWarps * sizeof(PathPool);
   size_t smem = pools + (kStage ? align16(maj_bytes) : 0u) + (kBatch ? bt.count * sizeof(BatchView) : 0u);
@@ -658,15 +660,15 @@ static vcr_status launch_t(vcr_ctx* ctx, const GridView& g, const SceneView& s, 
   return VCR_OK;
 }
 
-template <bool kBatch>
+template <bool kBatch, bool kCache>
 static vcr_status launch_b(vcr_ctx* ctx, const GridView& g, const SceneView& s, const CamView& cam,
                            const PassView& pv, uint32_t* stats, Counters cnt, uint32_t total, uint32_t bytes,
                            bool stage, const NrcTrainSink& ts, const BatchSink& bt, double* sum, cudaStream_t st) {
   if (ctx->tuning.block_threads == 128)
-    return stage ? launch_t<128, true, kBatch>(ctx, g, s, cam, pv, stats, cnt, total, bytes, ts, bt, sum, st)
-                 : launch_t<128, false, kBatch>(ctx, g, s, cam, pv, stats, cnt, total, bytes, ts, bt, sum, st);
-  return stage ? launch_t<256, true, kBatch>(ctx, g, s, cam, pv, stats, cnt, total, bytes, ts, bt, sum, st)
-               : launch_t<256, false, kBatch>(ctx, g, s, cam, pv, stats, cnt, total, bytes, ts, bt, sum, st);
+    return stage ? launch_t<128, true, kBatch, kCache>(ctx, g, s, cam, pv, stats, cnt, total, bytes, ts, bt, sum, st)
+                 : launch_t<128, false, kBatch, kCache>(ctx, g, s, cam, pv, stats, cnt, total, bytes, ts, bt, sum, st);
+  return stage ? launch_t<256, true, kBatch, kCache>(ctx, g, s, cam, pv, stats, cnt, total, bytes, ts, bt, sum, st)
+               : launch_t<256, false, kBatch, kCache>(ctx, g, s, cam, pv, stats, cnt, total, bytes, ts, bt, sum, st);
 }
 
 vcr_status wavefront_launch(vcr_ctx* ctx, const GridView& g, const SceneView& s, const CamView& cam,
@@ -685,8 +687,14 @@ vcr_status wavefront_launch(vcr_ctx* ctx, const GridView& g, const SceneView& s,
   uint32_t bytes = (uint32_t)(((cells + 3) & ~(size_t)3) * sizeof(float));  // padded level: 16-byte multiple
   bool stage = t.stage_majorants && bytes <= max_staged_bytes(t.block_threads);
   if (!sum) sum = ctx->d_sum;
-  return batch ? launch_b<true>(ctx, g, s, cam, pv, stats, cnt, total, bytes, stage, ts, bt, sum, st)
-               : launch_b<false>(ctx, g, s, cam, pv, stats, cnt, total, bytes, stage, ts, bt, sum, st);
+  // a launch with neither queries nor training paths takes a kernel without
+  // their parts, whose shorter loop is fetched faster: 8 passes of 1920x1080
+  // 5.29 -> 4.98 ms, 12 views 7.49 -> 7.12, 64x64 pixels 192 -> 174 us with the
+  // call's host time (batches refuse the cache)
+  if (batch) return launch_b<true, false>(ctx, g, s, cam, pv, stats, cnt, total, bytes, stage, ts, bt, sum, st);
+  return s.nrc_events || ts.paths
+             ? launch_b<false, true>(ctx, g, s, cam, pv, stats, cnt, total, bytes, stage, ts, bt, sum, st)
+             : launch_b<false, false>(ctx, g, s, cam, pv, stats, cnt, total, bytes, stage, ts, bt, sum, st);
 }
 
 }  // namespace VCR_WF_NS
