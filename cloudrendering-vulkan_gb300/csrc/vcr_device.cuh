@@ -79,14 +79,17 @@ __device__ __forceinline__ uint32_t corner_cell(const GridView& g, uint32_t cx, 
   return (t << 9) + (cx & 7u) + ((cy & 7u) << 3) + ((cz & 7u) << 6);
 }
 
-__device__ __forceinline__ float trilinear(const GridView& g, f3 nrm) {
+// kCorners: from the corner blocks (which the caller knows to be there), or
+// from the bricks' texels.
+template <bool kCorners>
+__device__ __forceinline__ float trilinear_from(const GridView& g, f3 nrm) {
   float ux = nrm.x * (float)g.n[0] - 0.5f;
   float uy = nrm.y * (float)g.n[1] - 0.5f;
   float uz = nrm.z * (float)g.n[2] - 0.5f;
   float fx0 = floorf(ux), fy0 = floorf(uy), fz0 = floorf(uz);
   float tx = ux - fx0, ty = uy - fy0, tz = uz - fz0;
   int x0 = (int)fx0, y0 = (int)fy0, z0 = (int)fz0;
-  if (g.corners) {  // one 32-byte block holds the footprint: the same values, the same lerps
+  if (kCorners) {  // one 32-byte block holds the footprint: the same values, the same lerps
     const uint32_t cx = (uint32_t)(min(max(x0, -1), g.n[0] - 1) + 1);
     const uint32_t cy = (uint32_t)(min(max(y0, -1), g.n[1] - 1) + 1);
     const uint32_t cz = (uint32_t)(min(max(z0, -1), g.n[2] - 1) + 1);
@@ -158,9 +161,13 @@ __device__ __forceinline__ float trilinear(const GridView& g, f3 nrm) {
 // Normalised coordinates (p - b0) / (b1 - b0) as in sampleCloud
 // (PathTracer.comp:117), by multiplication with the box's reciprocal extent
 // (a GLSL division may be evaluated that way, within 2.5 ulp).
-__device__ __forceinline__ float density_at(const GridView& g, const SceneView& s, f3 p) {
+template <bool kCorners>
+__device__ __forceinline__ float density_from(const GridView& g, const SceneView& s, f3 p) {
   const f3 q = p - s.b0;
-  return trilinear(g, mk(q.x * s.iext.x, q.y * s.iext.y, q.z * s.iext.z));
+  return trilinear_from<kCorners>(g, mk(q.x * s.iext.x, q.y * s.iext.y, q.z * s.iext.z));
+}
+__device__ __forceinline__ float density_at(const GridView& g, const SceneView& s, f3 p) {
+  return g.corners ? density_from<true>(g, s, p) : density_from<false>(g, s, p);
 }
 
 #endif  // __CUDACC__
