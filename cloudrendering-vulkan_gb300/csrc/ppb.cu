@@ -1115,7 +1115,7 @@ __global__ void __launch_bounds__(kGatherThreads, 6) ppb_gather_kernel(const __g
               }
             }
             const uint32_t peers = __match_any_sync(0xffffffffu, key);
-            if (lane < m && (peers & lt) == 0u) w.own[key] = peers;
+            if (key < 32u && (peers & lt) == 0u) w.own[key] = peers;  // a pixel: not a lane without a pair
             w.c[0][lane] = c.x;
             w.c[1][lane] = c.y;
             w.c[2][lane] = c.z;
