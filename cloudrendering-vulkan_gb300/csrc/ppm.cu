@@ -505,6 +505,7 @@ __global__ void __launch_bounds__(kPpmGatherThreads, 8)
           ++lev;
           next = w.next[lev];
           count = w.count[lev];
+          __syncwarp();  // before lane 0 writes them again
           continue;
         }
         if (lev > 0) {
