@@ -475,7 +475,7 @@ static vcr_status grid_finish(vcr_ctx* ctx, const vcr_grid_desc* desc, int preci
   ctx->gdesc = *desc;
   ctx->precision = precision;
   for (int a = 0; a < 3; ++a) ctx->nb[a] = nb[a];
-  unsigned int* d_gmax = reinterpret_cast<unsigned int*>(ctx->d_counters + 5);
+  unsigned int* d_gmax = reinterpret_cast<unsigned int*>(ctx->d_counters + kGridMaxCounter);
   VCR_CUDA(ctx, cudaMemsetAsync(d_gmax, 0, sizeof(unsigned int), s));
   const float* summary = reinterpret_cast<const float*>(ctx->d_scratch);
   majorant_from_summary_kernel<<<(unsigned)((nbricks + 255) / 256), 256, 0, s>>>(summary, nb[0], nb[1], nb[2],

@@ -1016,7 +1016,7 @@ static vcr_status nrc_launch_training(vcr_ctx* ctx, const PassView& pv, uint32_t
   NrcTrainSink ts = nrc_sink(ctx);
   ts.paths = paths;
   VCR_CUDA(ctx, cudaMemsetAsync(ts.count, 0, 4, s));
-  VCR_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0, 7 * sizeof(unsigned long long), s));
+  VCR_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0, kPassCounterBytes, s));
   return wavefront_launch(ctx, grid_view(ctx), scene_view(ctx), cam_view(ctx->cam), pv, nullptr,
                           Counters{ctx->d_counters}, 0u, s, &ts);
 }

@@ -28,8 +28,11 @@ struct PassView {
 };
 
 struct Counters {
-  unsigned long long* c;  // [0] paths [1] lookups [2] events [3] cells [4] cursor
+  unsigned long long* c;  // [0] paths [1] lookups [2] events [3] cells [4], [5] cursors
 };
+constexpr uint32_t kWorkCursor = 4, kTrainCursor = 5;
+constexpr size_t kPassCounterBytes = 6 * sizeof(unsigned long long);  // what a pass clears
+static_assert(kWorkCursor < 6 && kTrainCursor < 6 && kGridMaxCounter >= 6, "a pass clears its words, and no others");
 
 // ---------------------------------------------------------------------------
 // shared helpers

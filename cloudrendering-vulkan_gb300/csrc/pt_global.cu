@@ -153,7 +153,7 @@ vcr_status pt_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t 
   CamView cam = cam_view(ctx->cam);
   uint32_t* stats = (pv.flags & VCR_PASS_RECORD_STATS) ? ctx->d_stats : nullptr;
   Counters cnt{ctx->d_counters};
-  VCR_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0, 7 * sizeof(unsigned long long), st));
+  VCR_CUDA(ctx, cudaMemsetAsync(ctx->d_counters, 0, kPassCounterBytes, st));
   if (P.tracker == VCR_TRACKER_GLOBAL) {
     SvView sv{};
     if (ctx->has_sv) {

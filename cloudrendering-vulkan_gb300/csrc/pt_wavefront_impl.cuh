@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
           // ---- new paths ----------------------------------------------------
           const uint32_t take = min(min(n_free, cap), 32u);
           uint32_t base = 0;
-          if (lane == 0) base = (uint32_t)atomicAdd(cnt.c + (serving ? 6 : 4), (unsigned long long)take);
+          if (lane == 0) base = (uint32_t)atomicAdd(cnt.c + (serving ? kTrainCursor : kWorkCursor), (unsigned long long)take);
           base = __shfl_sync(0xffffffffu, base, 0) + (serving || !kCache || !train_warps ? 0u : n_train);
           const uint32_t end = serving ? n_train : total + n_train;
           exhausted = base + take >= end;

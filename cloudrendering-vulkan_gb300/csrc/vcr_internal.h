@@ -79,7 +79,8 @@ struct vcr_ctx {
   vcr::UploadStreams upload;
 
   // device counters: [0] paths [1] lookups [2] events [3] dda cells [4] work cursor
-  // [5] grid max (u32 bits) [6] training-path cursor [7] relRMSE accumulator (double bits)
+  // [5] training-path cursor [6] grid max (u32 bits) [7] relRMSE accumulator (double bits);
+  // a pass clears [0 .. 5] on its own stream, so the others are none of its words
   unsigned long long* d_counters = nullptr;
   int* d_error = nullptr;  // device error word (bounded waits, index checks)
 
@@ -141,6 +142,8 @@ __device__ __forceinline__ void warp_count(unsigned long long* dst, uint32_t v) 
 
 // Scratch buffer owned by the context (grown, never shrunk).
 vcr_status ensure_scratch(vcr_ctx* ctx, size_t bytes);
+
+constexpr uint32_t kGridMaxCounter = 6;  // of vcr_ctx::d_counters
 
 GridView grid_view(const vcr_ctx* ctx);
 SceneView scene_view(const vcr_ctx* ctx);
