@@ -216,12 +216,14 @@ constexpr int kThreadsPerSm = 768;
 constexpr uint32_t kRefillAt = 10;
 // Training paths run to their end (64 events) where camera paths of the
 // cached tracker end at their second event: each is a chain of dependent
-// steps, and the longest decides when the launch ends.  They start in warps
-// of their own, few a warp, which take camera paths only when theirs are
-// done, so that a step of theirs is short and nothing waits for 32 others.
-// 45 k of them with 4.1 M camera paths: 1,213 us a frame with mixed warps,
-// 976 at 8 to 32 a warp, 1,020 at 96.
-constexpr uint32_t kTrainPerWarp = 16;
+// steps, and the longest decides when the launch ends.  So they come first,
+// and apart from camera paths: one warp for every kTrainShare of them starts
+// on the training paths' own cursor, takes 32 neighbouring ones at a time like
+// any warp (a pool's worth in all, so that some of these warps find none
+// left), and camera paths once the cursor has run out.  45 k of them with
+// 4.1 M camera paths: 1,213 us a frame with mixed warps, 976 with a warp for
+// every 8 to 32, 1,020 for every 96.
+constexpr uint32_t kTrainShare = 16;
 // The paths a warp holds, in shared memory: the lanes fly 32 of them at a
 // time, the others wait in one of the queues.  With 80 the parts ran at 15
 // to 19 lanes and the passes above took 3 % longer; 128 leave two CTAs an SM.
@@ -652,7 +654,7 @@ static vcr_status launch_t(vcr_ctx* ctx, const GridView& g, const SceneView& s, 
   // with one path runs only that path's parts (64x64 pixels: 166 -> 126 us)
   uint32_t cap = (uint32_t)std::min<uint64_t>((paths + (uint64_t)blocks * kWarps - 1) / ((uint64_t)blocks * kWarps), 32u);
   blocks = std::min<uint32_t>(blocks, (uint32_t)((paths + (uint64_t)cap * kWarps - 1) / ((uint64_t)cap * kWarps)));
-  const uint32_t train_warps = cap == 32u && total ? (ts.paths + kTrainPerWarp - 1u) / kTrainPerWarp : 0u;
+  const uint32_t train_warps = cap == 32u && total ? (ts.paths + kTrainShare - 1u) / kTrainShare : 0u;
   NrcSink nq{nullptr, nullptr, 0u};
   if (s.nrc_events && ctx->nrc) nq = NrcSink{ctx->nrc->query, ctx->nrc->query_count, ctx->nrc->query_capacity};
   kern<<<blocks, kThreads, smem, st>>>(g, s, cam, pv, sum, stats, cnt, total, ctx->tuning.dda_steps, cap, train_warps, maj_bytes,
