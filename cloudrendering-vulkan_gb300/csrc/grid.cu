@@ -84,6 +84,17 @@ __device__ __forceinline__ void store_summary(const float (&v)[2][8], int lane, 
   }
 }
 
+// Sets *word if a texel of the warp's brick is below zero or not a number:
+// such a grid's majorants, zero at least, do not bound what a lookup gives.
+__device__ __forceinline__ void note_below_zero(const float (&v)[2][8], int lane, unsigned int* __restrict__ word) {
+  bool any = false;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int x = 0; x < 8; ++x) any = any || !(v[h][x] >= 0.0f);
+  if (__any_sync(0xffffffffu, any) && lane == 0) *word = 1u;
+}
+
 // One warp per brick (8 bricks per 256-thread CTA): lane l holds texel rows
 // l and l + 32 of the brick (row r = y + 8 z, 8 texels along x, zero
 // outside the grid), the warp's maximum is the brick's scale, and each row
@@ -100,7 +111,8 @@ __global__ void __launch_bounds__(kBrickWarps * 32) brick_kernel(const float* __
                                                                  void* __restrict__ bricks,
                                                                  float* __restrict__ scales, int nx, int ny, int nz,
                                                                  int bx, int by, uint32_t b0, uint32_t count,
-                                                                 int kb0, float* __restrict__ summary) {
+                                                                 int kb0, float* __restrict__ summary,
+                                                                 unsigned int* __restrict__ below_zero) {
   const uint32_t local = blockIdx.x * kBrickWarps + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (local >= count) return;  // warp-uniform
@@ -136,6 +148,7 @@ __global__ void __launch_bounds__(kBrickWarps * 32) brick_kernel(const float* __
       dst[0] = make_float4(v[h][0], v[h][1], v[h][2], v[h][3]);
       dst[1] = make_float4(v[h][4], v[h][5], v[h][6], v[h][7]);
     }
+    note_below_zero(v, lane, below_zero);
     store_summary(v, lane, summary + (size_t)b * 27);
     return;
   }
@@ -163,6 +176,7 @@ __global__ void __launch_bounds__(kBrickWarps * 32) brick_kernel(const float* __
     *reinterpret_cast<uint4*>(base16) = make_uint4(w[0], w[1], w[2], w[3]);
   }
   if (lane == 0) scales[b] = s;
+  note_below_zero(v, lane, below_zero);
   store_summary(v, lane, summary + (size_t)b * 27);
 }
 
@@ -436,6 +450,7 @@ static vcr_status grid_alloc(vcr_ctx* ctx, const vcr_grid_desc* desc, int precis
   if (st) return st;
   VCR_CUDA(ctx, cudaMemsetAsync(ctx->d_majorants, 0, mtotal * sizeof(float), s));
   VCR_CUDA(ctx, cudaMemsetAsync(ctx->d_scales, 0, nbricks * sizeof(float), s));
+  VCR_CUDA(ctx, cudaMemsetAsync(ctx->d_counters + kGridMaxCounter, 0, sizeof(unsigned long long), s));
   return VCR_OK;
 }
 
@@ -452,15 +467,16 @@ static vcr_status brick_launch(vcr_ctx* ctx, const float* dense, const vcr_grid_
   const unsigned blocks = (count + kBrickWarps - 1) / kBrickWarps;
   if (count == 0) return VCR_OK;
   float* summary = reinterpret_cast<float*>(ctx->d_scratch);
+  unsigned int* below_zero = reinterpret_cast<unsigned int*>(ctx->d_counters + kGridMaxCounter) + 1;
   if (precision == 0)
     brick_kernel<0><<<blocks, kBrickWarps * 32, 0, s>>>(dense, ctx->d_bricks, ctx->d_scales, n[0], n[1], n[2], bx,
-                                                         by, b0, count, kb0, summary);
+                                                         by, b0, count, kb0, summary, below_zero);
   else if (precision == 1)
     brick_kernel<1><<<blocks, kBrickWarps * 32, 0, s>>>(dense, ctx->d_bricks, ctx->d_scales, n[0], n[1], n[2], bx,
-                                                         by, b0, count, kb0, summary);
+                                                         by, b0, count, kb0, summary, below_zero);
   else
     brick_kernel<2><<<blocks, kBrickWarps * 32, 0, s>>>(dense, ctx->d_bricks, ctx->d_scales, n[0], n[1], n[2], bx,
-                                                         by, b0, count, kb0, summary);
+                                                         by, b0, count, kb0, summary, below_zero);
   VCR_CUDA(ctx, cudaGetLastError());
   return VCR_OK;
 }
@@ -476,7 +492,6 @@ static vcr_status grid_finish(vcr_ctx* ctx, const vcr_grid_desc* desc, int preci
   ctx->precision = precision;
   for (int a = 0; a < 3; ++a) ctx->nb[a] = nb[a];
   unsigned int* d_gmax = reinterpret_cast<unsigned int*>(ctx->d_counters + kGridMaxCounter);
-  VCR_CUDA(ctx, cudaMemsetAsync(d_gmax, 0, sizeof(unsigned int), s));
   const float* summary = reinterpret_cast<const float*>(ctx->d_scratch);
   majorant_from_summary_kernel<<<(unsigned)((nbricks + 255) / 256), 256, 0, s>>>(summary, nb[0], nb[1], nb[2],
                                                                                 ctx->d_majorants, d_gmax);
@@ -489,13 +504,14 @@ static vcr_status grid_finish(vcr_ctx* ctx, const vcr_grid_desc* desc, int preci
   const uint32_t cells3 = (uint32_t)(pv.n[3][0] * pv.n[3][1] * pv.n[3][2]);
   majorant_pyramid_kernel<<<(cells3 + 3) / 4, 128, 0, s>>>(ctx->d_majorants, pv, cells3);
   VCR_CUDA(ctx, cudaGetLastError());
-  unsigned int gm = 0;
-  VCR_CUDA(ctx, cudaMemcpyAsync(&gm, d_gmax, sizeof(gm), cudaMemcpyDeviceToHost, s));
+  unsigned int gm[2] = {0, 0};  // the maximum; whether there is a texel below zero
+  VCR_CUDA(ctx, cudaMemcpyAsync(gm, d_gmax, sizeof(gm), cudaMemcpyDeviceToHost, s));
   VCR_CUDA(ctx, cudaStreamSynchronize(s));
   float f;
-  memcpy(&f, &gm, sizeof(f));
+  memcpy(&f, gm, sizeof(f));
   if (!(f <= 3.0e38f)) return fail(ctx, VCR_ERR_INVALID, "grid holds non-finite densities");
   ctx->max_density = f;
+  ctx->below_zero = gm[1] != 0u;
   ctx->has_grid = true;
   if (ctx->tuning.corner_blocks && !corners_built) {
     vcr_status cs = corner_build(ctx, s);

@@ -296,7 +296,8 @@ __device__ __forceinline__ void warp_box(float4& lo, float4& hi) {
 // transmittance distances has none of them left, and where every majorant
 // cell its box touches is zero the density at the closest point is; both
 // factors of the estimate are then exactly 0.  A cell's majorant bounds the
-// trilinear lookups inside it.  The points looked up lie within the radius of
+// trilinear lookups inside it, unless the grid has texels below zero (or that
+// are no number): then every leaf is live.  The points looked up lie within the radius of
 // the segment; its box is grown by that, and by a hundredth of a cell against
 // the rounding of the cell index.
 struct LiveView {
@@ -305,7 +306,7 @@ struct LiveView {
   const float4* seg_b;
   const uint32_t* seg_beam;
   const float* reach;
-  const float* maj;  // a pyramid level
+  const float* maj;  // a pyramid level, or nullptr: every leaf is live
   int mnb[3];
   f3 b0, icell;
 };
@@ -338,7 +339,7 @@ __global__ void __launch_bounds__(256) ppb_live_kernel(const __grid_constant__ L
   if (i < n) {
     const uint32_t sid = v.order[i];
     const float4 B = v.seg_b[sid];
-    live = v.reach[v.seg_beam[sid]] >= B.w && segment_meets_density(v, v.seg_a[sid], B);
+    live = !v.maj || (v.reach[v.seg_beam[sid]] >= B.w && segment_meets_density(v, v.seg_a[sid], B));
   }
   const uint32_t m = __ballot_sync(0xffffffffu, live);
   if (lane == 0) {
@@ -564,6 +565,7 @@ struct PpbGatherView {
   float* cam_dist;
   ClusterLayout cl;
   float radius;
+  bool every_pair;  // not without the pairs that give exactly 0: the grid may hold texels that are no number
   uint32_t seed, pass;
 };
 
@@ -956,7 +958,7 @@ __global__ void __launch_bounds__(kGatherThreads, 6) ppb_gather_kernel(const __g
       // past the farthest flight (d[3].w) the camera transmittance is 0 (the
       // margin is over the rounding of t - t_in); the boxes are looked for
       // some radii further, as a closest point may lie before its box
-      const float t_far = fminf(t_out, (t_in + d[kBeamDists / 4 - 1].w) * 1.0001f);
+      const float t_far = v.every_pair ? t_out : fminf(t_out, (t_in + d[kBeamDists / 4 - 1].w) * 1.0001f);
       const float t_box = fminf(t_out, t_far + 8.0f * v.radius);
       depth = fmaf(view.W.x, fmaf(t_box, rd.x, o.x - view.apex.x),
                    fmaf(view.W.y, fmaf(t_box, rd.y, o.y - view.apex.y),
@@ -1368,7 +1370,7 @@ vcr_status ppb_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
                 ext.z / (float)ctx->gdesc.size[2] * voxels);
       if (level == 3 || std::min(cell.x, std::min(cell.y, cell.z)) >= 2.0f * st->radius) break;
     }
-    lv.maj = ctx->d_majorants + ctx->moff[level];
+    if (!ctx->below_zero) lv.maj = ctx->d_majorants + ctx->moff[level];
     for (int a = 0; a < 3; ++a) lv.mnb[a] = ctx->mnb[level][a];
     lv.icell = mk(1.0f / cell.x, 1.0f / cell.y, 1.0f / cell.z);
     const uint32_t c = (n + 31u) / 32u;
@@ -1390,6 +1392,7 @@ vcr_status ppb_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
   }
   gv.slots = st->slots;
   gv.radius = st->radius;
+  gv.every_pair = ctx->below_zero;
   gv.cluster_lo = st->cluster_lo;
   gv.cluster_hi = st->cluster_hi;
   vcr_status ps = probe_begin(ctx, st->gather, st_);

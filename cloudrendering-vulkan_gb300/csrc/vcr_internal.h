@@ -41,6 +41,7 @@ struct vcr_ctx {
   float* d_majorants = nullptr;  // pyramid levels 0..3, each 16-byte aligned
   size_t grid_bytes[3] = {0, 0, 0};  // allocated bytes of bricks, scales, majorants (kept for a same-size grid)
   float max_density = 0.0f;
+  bool below_zero = false;  // the grid has texels below zero (or that are no number)
   int nb[3] = {0, 0, 0};
   int mnb[4][3] = {};            // cells per axis of each majorant level
   size_t moff[4] = {};           // float offset of each level in d_majorants
@@ -79,8 +80,9 @@ struct vcr_ctx {
   vcr::UploadStreams upload;
 
   // device counters: [0] paths [1] lookups [2] events [3] dda cells [4] work cursor
-  // [5] training-path cursor [6] grid max (u32 bits) [7] relRMSE accumulator (double bits);
-  // a pass clears [0 .. 5] on its own stream, so the others are none of its words
+  // [5] training-path cursor [6] grid max (u32 bits, and in the upper half
+  // whether a texel is below zero) [7] relRMSE accumulator (double bits); a pass
+  // clears [0 .. 5] on its own stream, so the others are none of its words
   unsigned long long* d_counters = nullptr;
   int* d_error = nullptr;  // device error word (bounded waits, index checks)
 
