@@ -278,7 +278,8 @@ __global__ void dda_trace_kernel(SceneView s, int nc0, int nc1, int nc2, const f
   if (slab(org, dir, s.b0, s.b1, tmin, tmax) && tmax >= 0.0f) {
     if (tmin > 0.0f) {
       org = along(org, dir, tmin);
-      slab(org, dir, s.b0, s.b1, tmin, tmax);
+      // (at an edge the moved ray may miss by a rounding: the walk goes to where the test had got)
+      slab_inv(org, recip(dir), s.b0, s.b1, tmin, tmax, true);
     }
     Dda dd;
     dda_init(dd, org, dir, recip(dir), s.b0, s.cell, s.icell, nc);
