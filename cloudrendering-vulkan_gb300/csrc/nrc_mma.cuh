@@ -53,13 +53,6 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const void* p) {
                : "r"(a)
                : "memory");
 }
-__device__ __forceinline__ void ldsm_x2_t(uint32_t (&r)[2], const void* p) {
-  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
-               : "=r"(r[0]), "=r"(r[1])
-               : "r"(a)
-               : "memory");
-}
 
 // Global [in][out] BF16 weights (ld = cols) into the padded shared layout,
 // 16 bytes at a time by a CTA of kThreads threads: all of a thread's loads

@@ -146,12 +146,6 @@ __device__ __noinline__ PathStart start_path(const CamView& cam, const SceneView
   o.hit = true;
   return o;
 }
-__device__ __forceinline__ bool begin(const PathStart& o, f3& pos, f3& dir, f3& L) {
-  pos = o.pos;
-  dir = o.dir;
-  L = o.L;
-  return o.hit;
-}
 
 // A training path's radiance is final: turn the recorded radiance-before
 // and throughput-before of each of its vertices into the target

@@ -191,6 +191,14 @@ __device__ __forceinline__ uint2 scan256(uint32_t x, uint32_t y, uint32_t* sums)
   return r;
 }
 
+// A load that stays where it is written: moved up before the ranking, as the
+// compiler likes to, the values' registers push others to the stack.
+__device__ __forceinline__ uint32_t load_here(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
 // One digit pass over tiles of kT x kI keys (tile ids in launch order from an
 // atomic counter).  Warp w ranks the tile's keys [32 kI w, 32 kI (w + 1));
 // then one thread a digit: the exclusive prefix over the warps, the tile's
@@ -206,14 +214,7 @@ __device__ __forceinline__ uint2 scan256(uint32_t x, uint32_t y, uint32_t* sums)
 // share a bank in each of the counting, staging and base reads) and the
 // ballots' issue (42 %); leaving the look-back out gave 15 %, storing in
 // input order instead of scattered nothing.
-// A load that stays where it is written: moved up before the ranking, as the
-// compiler likes to, the values' registers push others to the stack.
-__device__ __forceinline__ uint32_t load_here(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-}
-
+//
 // kFull: every key of the tile exists.
 template <int kT, int kI, int kAhead, bool kFull>
 __device__ __forceinline__ void sort_tile(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
