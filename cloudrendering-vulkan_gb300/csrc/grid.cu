@@ -455,8 +455,8 @@ static vcr_status grid_alloc(vcr_ctx* ctx, const vcr_grid_desc* desc, int precis
   return VCR_OK;
 }
 
-// The summaries of a grid's bricks at the start of the scratch buffer, and
-// `extra` bytes behind them (ensure_scratch for what follows).
+// Bytes of the summaries of a grid's bricks, at the start of the scratch buffer
+// (an upload's ring may follow them).
 static size_t summary_bytes(uint64_t nbricks) { return ((size_t)nbricks * 27 * sizeof(float) + 255) & ~(size_t)255; }
 
 // Bricks [b0, b0 + count) and their summaries from `dense`, which holds z
@@ -482,8 +482,9 @@ static vcr_status brick_launch(vcr_ctx* ctx, const float* dense, const vcr_grid_
   return VCR_OK;
 }
 
-// Once every brick and summary is written: majorant pyramid, global maximum, and the corner blocks unless the caller built them already
-// (synchronises on s).
+// Once every brick and summary is written: majorant pyramid, global maximum,
+// and the corner blocks unless the caller built them already (synchronises on
+// s).
 static vcr_status grid_finish(vcr_ctx* ctx, const vcr_grid_desc* desc, int precision, cudaStream_t s,
                               bool corners_built = false) {
   int nb[3];

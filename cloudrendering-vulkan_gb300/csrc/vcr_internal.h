@@ -151,7 +151,7 @@ GridView grid_view(const vcr_ctx* ctx);
 SceneView scene_view(const vcr_ctx* ctx);
 
 // grid.cu
-// A host grid, uploaded and bricked one brick layer at a time.
+// A host grid, uploaded and bricked a slab of brick layers at a time.
 vcr_status grid_upload_host(vcr_ctx* ctx, const float* host, const vcr_grid_desc* desc, int precision);
 void upload_free(vcr_ctx* ctx);
 vcr_status grid_build(vcr_ctx* ctx, const float* d_dense, const vcr_grid_desc* desc, int precision,

@@ -179,7 +179,9 @@ typedef struct vcr_shadow_volume {
 typedef struct vcr_tuning {
   uint32_t majorant_level;  /* 0..3 */
   uint32_t dda_steps;       /* majorant cells a lane may walk per wavefront step, >= 1 */
-  uint32_t stage_majorants; /* 1: stage the level's majorants in shared memory (TMA bulk copy) when they fit */
+  uint32_t stage_majorants; /* 1: stage the level's majorants in shared memory (TMA bulk copy) when they fit
+                               beside the paths a CTA holds there: up to 64 bytes a thread, 16 KB (4,096 cells)
+                               at 256 threads, 8 KB at 128; larger levels are read through the L1 */
   uint32_t block_threads;   /* wavefront CTA size: 128 or 256 */
   uint32_t corner_blocks;   /* 1 (default): density lookups read a per-cell block of the 8 decoded trilinear
                                corners (32 bytes, one sector) built from the bricks, 32 B per voxel of device
@@ -582,8 +584,8 @@ VCR_API vcr_status vcr_ppb_setup(vcr_ctx* ctx, const vcr_ppb_params* p);
 VCR_API vcr_status vcr_ppb_free(vcr_ctx* ctx);
 /* One progressive pass (RecordDrawCommands, RenderTechniquePPB.cpp:436-519):
  * photon emission with beam deposit (PPB_PT.comp), segmenting + 30-bit
- * Morton keys, radix sort, LBVH build (PPB_GenerateHierarchy.comp), AABB
- * refit (PPB_CalculateAABB.comp), per-pixel beam gather (PPB_PE.comp); the
+ * Morton keys, radix sort, LBVH build (PPB_GenerateHierarchy.comp) and its
+ * boxes (PPB_CalculateAABB.comp), per-pixel beam gather (PPB_PE.comp); the
  * radius of pass k is r0 prod_{i=1..k} (i + alpha)/(i + 1) (UpdateRadius,
  * :530-546).  One estimate per pixel is added to the FP64 sums. */
 VCR_API vcr_status vcr_ppb_pass(vcr_ctx* ctx, const vcr_pass_desc* pass, void* stream);
@@ -591,7 +593,8 @@ VCR_API vcr_status vcr_ppb_info(vcr_ctx* ctx, vcr_ppb_info_t* out);
 /* The last pass's gather: (pixel, beam segment) pairs it evaluated (segments
  * of which a point may come within the radius of the pixel's ray, without
  * those that contribute exactly 0: past the beam's or the camera ray's
- * farthest transmittance sample, or in cells without density) and its device
+ * farthest transmittance sample, or in cells without density; a grid with
+ * texels below zero leaves none out) and its device
  * time (the camera rays' samples are drawn with the beams, before it).  Waits
  * for the gather to finish.  No reference counterpart
  * (measurement). */
@@ -599,8 +602,9 @@ VCR_API vcr_status vcr_ppb_gather_stats(vcr_ctx* ctx, uint64_t* segments_evaluat
 /* Synchronous copy of one of the last pass's beam buffers. */
 VCR_API vcr_status vcr_ppb_read(vcr_ctx* ctx, vcr_ppb_buffer which, void* host_out, size_t bytes);
 /* LBVH over n Morton-sorted segments (device buffers): Karras build with
- * index-augmented prefixes for equal keys, then capped-cylinder leaf boxes
- * and the bottom-up refit.  d_order[i] = segment of sorted leaf i;
+ * index-augmented prefixes for equal keys, capped-cylinder leaf boxes, and
+ * each node's box from the leaf boxes of its range (the boxes of a bottom-up
+ * refit).  d_order[i] = segment of sorted leaf i;
  * segments are float4 (start, radius) and float4 (end, any).  Internal node
  * children carry bit 31 for leaves.  Replaces PPB_GenerateHierarchy.comp
  * (:122-168) + PPB_CalculateAABB.comp (:100-120). */
