@@ -447,11 +447,11 @@ static vcr_status grid_alloc(vcr_ctx* ctx, const vcr_grid_desc* desc, int precis
   // the previous grid's buffers are kept where their sizes match
   vcr_status st = grid_buffer(ctx, &ctx->d_bricks, ctx->grid_bytes[0], nbricks * kBrickVoxels * esz);
   if (!st) st = grid_buffer(ctx, reinterpret_cast<void**>(&ctx->d_scales), ctx->grid_bytes[1], nbricks * sizeof(float));
-  if (!st) st = grid_buffer(ctx, reinterpret_cast<void**>(&ctx->d_majorants), ctx->grid_bytes[2], mtotal * sizeof(float));
+  if (!st) st = grid_buffer(ctx, reinterpret_cast<void**>(&ctx->d_majorants), ctx->grid_bytes[2], (mtotal + 4) * sizeof(float));
   if (st) return st;
-  VCR_CUDA(ctx, cudaMemsetAsync(ctx->d_majorants, 0, mtotal * sizeof(float), s));
+  ctx->d_grid_max = reinterpret_cast<unsigned int*>(ctx->d_majorants + mtotal);
+  VCR_CUDA(ctx, cudaMemsetAsync(ctx->d_majorants, 0, (mtotal + 4) * sizeof(float), s));
   VCR_CUDA(ctx, cudaMemsetAsync(ctx->d_scales, 0, nbricks * sizeof(float), s));
-  VCR_CUDA(ctx, cudaMemsetAsync(ctx->d_counters + kGridMaxCounter, 0, sizeof(unsigned long long), s));
   return VCR_OK;
 }
 
@@ -468,7 +468,7 @@ static vcr_status brick_launch(vcr_ctx* ctx, const float* dense, const vcr_grid_
   const unsigned blocks = (count + kBrickWarps - 1) / kBrickWarps;
   if (count == 0) return VCR_OK;
   float* summary = reinterpret_cast<float*>(ctx->d_scratch);
-  unsigned int* below_zero = reinterpret_cast<unsigned int*>(ctx->d_counters + kGridMaxCounter) + 1;
+  unsigned int* below_zero = ctx->d_grid_max + 1;
   if (precision == 0)
     brick_kernel<0><<<blocks, kBrickWarps * 32, 0, s>>>(dense, ctx->d_bricks, ctx->d_scales, n[0], n[1], n[2], bx,
                                                          by, b0, count, kb0, summary, below_zero);
@@ -493,10 +493,9 @@ static vcr_status grid_finish(vcr_ctx* ctx, const vcr_grid_desc* desc, int preci
   ctx->gdesc = *desc;
   ctx->precision = precision;
   for (int a = 0; a < 3; ++a) ctx->nb[a] = nb[a];
-  unsigned int* d_gmax = reinterpret_cast<unsigned int*>(ctx->d_counters + kGridMaxCounter);
   const float* summary = reinterpret_cast<const float*>(ctx->d_scratch);
   majorant_from_summary_kernel<<<(unsigned)((nbricks + 255) / 256), 256, 0, s>>>(summary, nb[0], nb[1], nb[2],
-                                                                                ctx->d_majorants, d_gmax);
+                                                                                ctx->d_majorants, ctx->d_grid_max);
   VCR_CUDA(ctx, cudaGetLastError());
   PyramidView pv{};
   for (int l = 0; l < 4; ++l) {
@@ -507,7 +506,7 @@ static vcr_status grid_finish(vcr_ctx* ctx, const vcr_grid_desc* desc, int preci
   majorant_pyramid_kernel<<<(cells3 + 3) / 4, 128, 0, s>>>(ctx->d_majorants, pv, cells3);
   VCR_CUDA(ctx, cudaGetLastError());
   unsigned int gm[2] = {0, 0};  // the maximum; whether there is a texel below zero
-  VCR_CUDA(ctx, cudaMemcpyAsync(gm, d_gmax, sizeof(gm), cudaMemcpyDeviceToHost, s));
+  VCR_CUDA(ctx, cudaMemcpyAsync(gm, ctx->d_grid_max, sizeof(gm), cudaMemcpyDeviceToHost, s));
   VCR_CUDA(ctx, cudaStreamSynchronize(s));
   float f;
   memcpy(&f, gm, sizeof(f));

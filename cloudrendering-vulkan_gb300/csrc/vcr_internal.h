@@ -39,6 +39,7 @@ struct vcr_ctx {
   void* d_bricks = nullptr;
   float* d_scales = nullptr;
   float* d_majorants = nullptr;  // pyramid levels 0..3, each 16-byte aligned
+  unsigned int* d_grid_max = nullptr;  // behind them: the grid's maximum (float bits), whether a texel is below zero
   size_t grid_bytes[3] = {0, 0, 0};  // allocated bytes of bricks, scales, majorants (kept for a same-size grid)
   float max_density = 0.0f;
   bool below_zero = false;  // the grid has texels below zero (or that are no number)
@@ -80,9 +81,8 @@ struct vcr_ctx {
   vcr::UploadStreams upload;
 
   // device counters: [0] paths [1] lookups [2] events [3] dda cells [4] work cursor
-  // [5] training-path cursor [6] grid max (u32 bits, and in the upper half
-  // whether a texel is below zero) [7] relRMSE accumulator (double bits); a pass
-  // clears [0 .. 5] on its own stream, so the others are none of its words
+  // [5] training-path cursor [7] relRMSE accumulator (double bits); a pass clears
+  // [0 .. 5] on its own stream
   unsigned long long* d_counters = nullptr;
   int* d_error = nullptr;  // device error word (bounded waits, index checks)
 
@@ -144,8 +144,6 @@ __device__ __forceinline__ void warp_count(unsigned long long* dst, uint32_t v) 
 
 // Scratch buffer owned by the context (grown, never shrunk).
 vcr_status ensure_scratch(vcr_ctx* ctx, size_t bytes);
-
-constexpr uint32_t kGridMaxCounter = 6;  // of vcr_ctx::d_counters
 
 GridView grid_view(const vcr_ctx* ctx);
 SceneView scene_view(const vcr_ctx* ctx);
